@@ -251,6 +251,32 @@ int rr_zscan_fused_opt(const rr_scan_targets* targets, const rr_scan_template* t
                        rr_stream_t stream);
 
 /* ------------------------------------------------------------------------
+ * Scan of a few targets: the same outputs for targets [first, first + count)
+ * (position block * 32 + lane of the packed targets) alone, a warp per
+ * (target, redshift) with the pixels over its lanes.  A fused-scan block
+ * costs the same with one target as with 32, so this is the path of small
+ * batches and of the last few targets of a batch; RR_SOLVE_NNLS and
+ * RR_SOLVE_BVLS (unbounded) templates run here at any count, with chi2 the
+ * direct residual.  y is summed in FP64 (y_ext is not read); a target's
+ * results do not depend on count.  basis_stride must be nbasis rounded up
+ * to even.
+ *   rr_few_rows_doubles  doubles of packed rows per target (-1: bad targets)
+ *   rr_pack_few          lrows[count][rr_few_rows_doubles] from targets->rw
+ *   rr_zscan_few         resweep: 2 device ints (caller zeroes) that count
+ *                        tiles and pairs summed again as the direct residual
+ *                        (PCA only), or NULL; after_fused != 0: the call
+ *                        before it on the stream was rr_zscan_fused, whose
+ *                        last tiles its launches may overlap (lrows must
+ *                        have been packed before that call).
+ * ---------------------------------------------------------------------- */
+int64_t rr_few_rows_doubles(const rr_scan_targets* targets);
+int rr_pack_few(const rr_scan_targets* targets, int64_t first, int32_t count, double* lrows,
+                rr_stream_t stream);
+int rr_zscan_few(const rr_scan_targets* targets, int64_t first, int32_t count,
+                 const double* lrows, const rr_scan_template* templates, int ntemplate,
+                 int* resweep, int after_fused, int* status, rr_stream_t stream);
+
+/* ------------------------------------------------------------------------
  * Pair scan: chi2, coefficients and penalty for an arbitrary list of
  * (target, redshift) pairs, the template rebinned (+ IGM) on the fly for
  * each pair -- the batched form of fitz's fine-grid refinement

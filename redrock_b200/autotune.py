@@ -60,10 +60,10 @@ def tune(pack, bases, repeats=1):
             continue
         times = {}
         for zt in cands:
-            run_fused(pack, sub, tiles={nb: zt})   # untimed (first launch of a variant)
+            run_fused(pack, sub, tiles={nb: zt}, tail=0)   # untimed (first launch of a variant)
             ev = []
             for _ in range(repeats):
-                run_fused(pack, sub, tiles={nb: zt}, kernel_events=ev)
+                run_fused(pack, sub, tiles={nb: zt}, kernel_events=ev, tail=0)
             torch.cuda.synchronize()
             times[zt] = sum(a.elapsed_time(b) for a, b in ev) / len(ev)
         best[nb] = min(times, key=times.get)
@@ -77,10 +77,10 @@ def tune(pack, bases, repeats=1):
         times = {}
         for g in groups:
             tiles = dict(zt, block_group=g)
-            run_fused(pack, sub, tiles=tiles)
+            run_fused(pack, sub, tiles=tiles, tail=0)
             ev = []
             for _ in range(repeats):
-                run_fused(pack, sub, tiles=tiles, kernel_events=ev)
+                run_fused(pack, sub, tiles=tiles, kernel_events=ev, tail=0)
             torch.cuda.synchronize()
             times[g] = sum(a.elapsed_time(b) for a, b in ev) / len(ev)
         best["block_group"] = min(times, key=times.get)

@@ -411,14 +411,16 @@ class TargetPack:
     def check(self):
         self._status.check("rr_pack_targets")
 
-    def scan_targets_struct(self):
+    def scan_targets_struct(self, nblock=None, rows=None):
         # one segment array per pack: every struct handed out points at it,
         # so it must outlive all of them
         if getattr(self, "_segarr", None) is None:
             self._segarr = (_lib.SegmentDesc * len(self.segs))(*self.segs)
         arr = self._segarr
-        return _lib.ScanTargets(ptr(self.rw), ptr(self.fwf), ptr(self.wsum), ptr(self.rows),
-                                ctypes.cast(arr, ctypes.c_void_p).value, self.nblock,
+        return _lib.ScanTargets(ptr(self.rw), ptr(self.fwf), ptr(self.wsum),
+                                ptr(self.rows if rows is None else rows),
+                                ctypes.cast(arr, ctypes.c_void_p).value,
+                                self.nblock if nblock is None else nblock,
                                 len(self.segs), self.npix_block)
 
 
@@ -438,20 +440,21 @@ class YGemm:
     on the DeviceBasis, rr_ygemm_i8), or the FP32-accumulated "bf16x3" /
     "tf32x3" (rr_ygemm)."""
 
-    def __init__(self, pack, variant, stream=None, status=None):
+    def __init__(self, pack, variant, stream=None, status=None, nblock=None):
         L = _lib.lib()
         dev = device()
         if variant not in _lib.YGEMM_VARIANTS or variant == "fp64":
             raise ValueError(f"unknown tensor-core y variant {variant!r}")
         self.variant = _lib.YGEMM_VARIANTS[variant]
         self.layout = pack.layout
-        self.npos = round_up(pack.nblock * _lib.LANES, 128)
+        nblock = pack.nblock if nblock is None else nblock
+        self.npos = round_up(nblock * _lib.LANES, 128)
         self.kpad = int(L.rr_ygemm_kpad(pack.layout.pix_stride))
         self.g = torch.empty((self.kpad, self.npos), dtype=torch.float64, device=dev)
         exact = self.variant in _lib.I8_VARIANTS
         self.row_exp = torch.empty(self.npos, dtype=torch.int32, device=dev) if exact else None
         self._status = status or StatusWord(dev)
-        tgs = pack.scan_targets_struct()
+        tgs = pack.scan_targets_struct(nblock)
         sh = stream_handle(stream)
         rc = L.rr_pack_g(ctypes.byref(tgs), pack.layout.pix_stride, self.kpad, self.npos,
                          ptr(self.g), ptr(self.row_exp), self._status.ptr, sh)
@@ -513,57 +516,127 @@ def _record(ev, stream):
         ev.record()
 
 
+# the last targets of a batch that do not fill a 32-target block of the
+# fused scan go through the few-target kernel when there are at most this
+# many of them: with all seven templates a target costs it 1.65 ms, a block
+# of the fused scan about 17 ms however many of its lanes are used (GALAXY
+# 10.5, QSO 4.4, STAR 2.6, measured at 37 targets)
+FEW_MAX = 10
+
+
+def few_tail(ntarget):
+    """How many of a batch's last targets the few-target kernel scans."""
+    t = ntarget % _lib.LANES
+    return t if t <= FEW_MAX else 0
+
+
+def _scan_templates(bases, results):
+    return [_lib.ScanTemplate(ptr(b.basis), b.layout.pix_stride, b.nz, b.nbasis, b.stride,
+                              b.method, ptr(b.prior), ptr(b.oii), ptr(r.zchi2), ptr(r.zcoeff),
+                              ptr(r.penalty) if b.oii is not None else None,
+                              ptr(getattr(r, "y_ext", None)))
+            for b, r in zip(bases, results)]
+
+
+class FewRows:
+    """The packed rows of a pack's targets first .. first + count - 1 for the
+    few-target kernel (rr_pack_few)."""
+
+    def __init__(self, pack, first, count, stream=None):
+        L = _lib.lib()
+        self.pack, self.first, self.count = pack, first, count
+        self.tgs = pack.scan_targets_struct()
+        n = int(L.rr_few_rows_doubles(ctypes.byref(self.tgs)))
+        if n < 0:
+            raise ValueError("target segments do not fit the few-target scan")
+        self.lrows = torch.empty(count * n, dtype=torch.float64, device=pack.rw.device)
+        rc = L.rr_pack_few(ctypes.byref(self.tgs), first, count, ptr(self.lrows),
+                           stream_handle(stream))
+        _lib.check(rc, "rr_pack_few")
+
+    def scan(self, bases, results, counter, status, after_fused=False, stream=None):
+        """chi2, coefficients and penalty of these targets into their rows
+        of the results (any solve method)."""
+        tms = _scan_templates(bases, results)
+        arr = (_lib.ScanTemplate * len(tms))(*tms)
+        rc = _lib.lib().rr_zscan_few(ctypes.byref(self.tgs), self.first, self.count,
+                                     ptr(self.lrows), arr, len(tms),
+                                     counter.data_ptr() + 2 * counter.element_size(),
+                                     int(after_fused), status.ptr, stream_handle(stream))
+        _lib.check(rc, "rr_zscan_few")
+
+
 def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=None,
-              tiles=None, external_events=False):
+              tiles=None, external_events=False, tail=None):
     """One persistent launch over every (target, template, z).  ygemm:
     None (DEFAULT_Y), "fp64", "int8x6", "int8x7", "bf16x3" or "tf32x3"; other than
     "fp64", y is computed on the tensor cores first (YGemm).  kernel_events:
     a list that gets a (start, end) CUDA event pair around the scan launches
     alone (timing).  tiles: redshifts per thread {nbasis: ZT} for the small
     bases (nbasis 4: 1-3, nbasis 5: 1-2; rr_scan_options) and optionally
-    "block_group" (the tile order), else the defaults."""
+    "block_group" (the tile order), else the defaults.  tail: how many of the
+    last targets go through the few-target kernel (FewRows) instead of the
+    fused one; None is few_tail's rule, or none when a y variant is asked
+    for."""
     L = _lib.lib()
     dev = device()
     results = [ScanResult(pack.ntarget, b, dev) for b in bases]
-    tgs = pack.scan_targets_struct()
+    for b in bases:
+        if b.layout.signature != pack.layout.signature:
+            raise ValueError("template basis and targets use different wavelength grids")
     counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=dev)
     st = status or StatusWord(dev)
-    ygemm = resolve_y(ygemm, pack.layout)
-    yg = None if ygemm == "fp64" else YGemm(pack, ygemm, stream=stream, status=st)
+    if tail is None:
+        plain_pca = all(b.method in (_lib.RR_SOLVE_PCA, _lib.RR_SOLVE_UNSUPPORTED)
+                        and b.stride == round_up(b.nbasis, 2) for b in bases)
+        tail = few_tail(pack.ntarget) if ygemm is None and plain_pca else 0
+    nfull = pack.ntarget - tail
+    few = FewRows(pack, nfull, tail, stream=stream) if tail else None
+    fused = nfull > 0 or not tail
+    rows = None
+    if fused:
+        nblock = max(1, (nfull + _lib.LANES - 1) // _lib.LANES)
+        if tail and nfull % _lib.LANES:
+            # the last fused block also holds targets of the tail: not its rows
+            rows = pack.rows.clone()
+            rows[nfull:] = -1
+        tgs = pack.scan_targets_struct(nblock, rows)
+        ygemm = resolve_y(ygemm, pack.layout)
+        yg = None if ygemm == "fp64" else YGemm(pack, ygemm, stream=stream, status=st,
+                                                nblock=nblock)
     for i0 in range(0, len(bases), _lib.MAX_TEMPLATES):
-        chunk = list(range(i0, min(len(bases), i0 + _lib.MAX_TEMPLATES)))
-        tms = []
-        for i in chunk:
-            b, r = bases[i], results[i]
-            if b.layout.signature != pack.layout.signature:
-                raise ValueError("template basis and targets use different wavelength grids")
+        sub = bases[i0:i0 + _lib.MAX_TEMPLATES]
+        out = results[i0:i0 + _lib.MAX_TEMPLATES]
+        if fused:
             if yg is not None:
-                # kept with the result so it outlives the launch
-                r.y_ext = yg.y(b, stream=stream)
-            tms.append(_lib.ScanTemplate(ptr(b.basis), b.layout.pix_stride, b.nz, b.nbasis,
-                                         b.stride, b.method, ptr(b.prior), ptr(b.oii),
-                                         ptr(r.zchi2), ptr(r.zcoeff),
-                                         ptr(r.penalty) if b.oii is not None else None,
-                                         ptr(r.y_ext) if yg is not None else None))
-        arr = (_lib.ScanTemplate * len(tms))(*tms)
-        if kernel_events is not None:
-            # external events become event-record nodes when the launches
-            # are captured in a CUDA graph, so each replay times them
-            e0 = torch.cuda.Event(enable_timing=True, external=external_events)
-            e1 = torch.cuda.Event(enable_timing=True, external=external_events)
-            _record(e0, stream)
-        if tiles:
-            opt = _lib.ScanOptions(int(tiles.get(4, 0)), int(tiles.get(5, 0)),
-                                   int(tiles.get("block_group", 0)))
-            rc = L.rr_zscan_fused_opt(ctypes.byref(tgs), arr, len(tms), ptr(counter),
-                                      ctypes.byref(opt), st.ptr, stream_handle(stream))
-        else:
-            rc = L.rr_zscan_fused(ctypes.byref(tgs), arr, len(tms), ptr(counter), st.ptr,
-                                  stream_handle(stream))
-        _lib.check(rc, "rr_zscan_fused")
-        if kernel_events is not None:
-            _record(e1, stream)
-            kernel_events.append((e0, e1))
+                for b, r in zip(sub, out):
+                    # kept with the result so it outlives the launch
+                    r.y_ext = yg.y(b, stream=stream)
+            tms = _scan_templates(sub, out)
+            arr = (_lib.ScanTemplate * len(tms))(*tms)
+            if kernel_events is not None:
+                # external events become event-record nodes when the launches
+                # are captured in a CUDA graph, so each replay times them
+                e0 = torch.cuda.Event(enable_timing=True, external=external_events)
+                e1 = torch.cuda.Event(enable_timing=True, external=external_events)
+                _record(e0, stream)
+            if tiles:
+                opt = _lib.ScanOptions(int(tiles.get(4, 0)), int(tiles.get(5, 0)),
+                                       int(tiles.get("block_group", 0)))
+                rc = L.rr_zscan_fused_opt(ctypes.byref(tgs), arr, len(tms), ptr(counter),
+                                          ctypes.byref(opt), st.ptr, stream_handle(stream))
+            else:
+                rc = L.rr_zscan_fused(ctypes.byref(tgs), arr, len(tms), ptr(counter), st.ptr,
+                                      stream_handle(stream))
+            _lib.check(rc, "rr_zscan_fused")
+            if kernel_events is not None:
+                _record(e1, stream)
+                kernel_events.append((e0, e1))
+        if few is not None:
+            few.scan(sub, out, counter, st, after_fused=fused and kernel_events is None,
+                     stream=stream)
+    for r in results[:1]:
+        r.few = (few, rows)   # outlive the launches
     run_fused.last_counter = counter
     return results, st
 

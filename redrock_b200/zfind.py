@@ -405,7 +405,7 @@ class DeviceFitzPlan:
         import torch
         from . import autotune
         from .device import StatusWord, to_device
-        from .engine import TargetBatch, TargetPack, TemplateSource
+        from .engine import TargetBatch, TargetPack, TemplateSource, few_tail, run_fused
         from .zscan import _bases_for
         self.local = local
         self.templates = list(templates)
@@ -421,7 +421,7 @@ class DeviceFitzPlan:
         self.rowpack = RowPack(self.dbatch)
         key = _PackShape(layout, self.dbatch.batch.nblock)
         best = autotune.choice(key, self.bases)
-        if best is None:
+        if best is None and few_tail(len(local)) < len(local):
             pack0 = TargetPack(self.dbatch, status=self.status)
             best = autotune.tune(pack0, self.bases)
             del pack0
@@ -433,7 +433,11 @@ class DeviceFitzPlan:
             # first 32 targets
             small = local[:32]
             wb = TargetBatch(small, layout).to_device()
-            wres = self._scan(wb)
+            wpack = TargetPack(wb, status=self.status)
+            # both scan kernels, whichever this batch's size needs
+            for tail in (len(small), 0):
+                wres, _ = run_fused(wpack, self.bases, status=self.status, tiles=self.tiles,
+                                    tail=tail)
             wrows = RowPack(wb)
             for k in range(len(self.templates)):
                 self._fine(k, wres[k], wrows)

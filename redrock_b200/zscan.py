@@ -17,7 +17,8 @@ DistTemplate's arrays in place, call ``clear_caches()``.  Error conventions foll
 rows with zero coefficients; an exactly singular normal matrix gives
 HUGE_CHI2 at that z; an unrecognised solve method gives HUGE_CHI2
 everywhere.  Non-negative / bounded solvers (NMF, NNLS, BVLS) run on the
-GPU too, through the plain chain's device solvers.
+GPU too: the scan in the few-target kernel, calc_zchi2_batch in the plain
+chain's device solvers.
 """
 
 from __future__ import annotations
@@ -29,8 +30,8 @@ import torch
 
 from . import _lib
 from .device import to_device, to_numpy
-from .engine import (DeviceBasis, GridLayout, IdCache, PlainTarget, ScanResult, TargetBatch,
-                     TargetPack, resolve_y, run_fused, run_plain)
+from .engine import (DeviceBasis, FewRows, GridLayout, IdCache, PlainTarget, ScanResult,
+                     TargetBatch, TargetPack, few_tail, resolve_y, run_fused, run_plain)
 from .templates import oii_sums, solve_code, solve_code_of
 
 HUGE_CHI2 = 9999999.0
@@ -117,6 +118,7 @@ CHUNK_TARGETS = 224   # targets per pipelined chunk (7 target blocks)
 LARGE_BATCH = 2048
 CHUNK_TARGETS_LARGE = 448
 AUTOTUNE = True       # time the small-basis tile shapes once per workload signature
+BOUNDED_CHUNK = 256   # targets per few-target launch of a bounded-solve template
 FIRST_CHUNK = 64      # a small first chunk gets the GPU started early
 # (64 / 224 measured best of 32-64 / 128-468 for 500 DESI-like targets:
 # 304.6 ms per end-to-end step against 315.3 ms for 32 / 128)
@@ -174,29 +176,58 @@ class HostResult:
 
 
 # solve methods the fused scan handles; NNLS / BVLS templates (their chi2 is
-# the direct residual of a bounded solve) go through the plain chain
+# the direct residual of a bounded solve) go through the few-target kernel
 _FUSED_METHODS = (_lib.RR_SOLVE_PCA, _lib.RR_SOLVE_UNSUPPORTED)
 
 
-def _plain_scan(targets, basis, layout):
-    """One template with a bounded solve: the plain per-target chain for
-    every target (calc_zchi2's loop, zscan.py:853-887), results on the
-    device like the fused scan's."""
+def _bounded_scan(targets, basis, layout):
+    """One template with a bounded solve (calc_zchi2's loop, zscan.py:853-887)
+    for every target, results on the device like the fused scan's: the
+    few-target kernel, BOUNDED_CHUNK targets at a time (their packed rows
+    take about 1 MB each).  Targets it cannot take -- a negative or NaN
+    weight, whose square root the packed rows hold, or more spectra on a
+    grid than a pack has segments for -- go through the plain per-target
+    chain."""
+    from .device import StatusWord
+    plain = [i for i, t in enumerate(targets)
+             if not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
+    few = [i for i in range(len(targets)) if i not in set(plain)]
     res = ScanResult(len(targets), basis, torch.device("cuda", torch.cuda.current_device()))
-    for i, t in enumerate(targets):
-        w = np.concatenate([s.ivar for s in t.spectra])
-        if w.sum() == 0:
-            res.zchi2[i] = HUGE_CHI2
-            res.zcoeff[i] = 0.0
+    st = StatusWord()
+    counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=res.zchi2.device)
+    for i0 in range(0, len(few), BOUNDED_CHUNK):
+        ix = few[i0:i0 + BOUNDED_CHUNK]
+        part = [targets[i] for i in ix]
+        try:
+            pack = _pack(part, layout) if len(ix) == len(targets) else \
+                TargetPack.from_targets(part, layout)
+        except NotImplementedError:
+            plain += ix
             continue
-        pt = PlainTarget(t.spectra, layout)
-        zc, co = run_plain(pt, basis, method=basis.method)
-        res.zchi2[i] = zc
-        res.zcoeff[i] = co
-        if basis.oii is not None:
-            res.penalty[i] = calc_negOII_penalty_sums(basis.oii, co)
-        pt._status.check("rr_zchi2_batch_plain_ex")
+        if len(ix) < len(targets):
+            pack.rows[:len(ix)] = torch.as_tensor(ix, dtype=torch.int32).to(pack.rows.device)
+        FewRows(pack, 0, len(ix)).scan([basis], [res], counter, st)
+        pack.check()
+    st.check("rr_zscan_few")
+    for i in plain:
+        _plain_target(targets[i], basis, layout, res, i)
     return res
+
+
+def _plain_target(t, basis, layout, res, i):
+    """Row i of a scan result through the plain per-target chain."""
+    w = np.concatenate([s.ivar for s in t.spectra])
+    if w.sum() == 0:
+        res.zchi2[i] = HUGE_CHI2
+        res.zcoeff[i] = 0.0
+        return
+    pt = PlainTarget(t.spectra, layout)
+    zc, co = run_plain(pt, basis, method=basis.method)
+    res.zchi2[i] = zc
+    res.zcoeff[i] = co
+    if basis.oii is not None:
+        res.penalty[i] = calc_negOII_penalty_sums(basis.oii, co)
+    pt._status.check("rr_zchi2_batch_plain_ex")
 
 
 def calc_negOII_penalty_sums(oii_sums_dev, coeff_t):
@@ -293,7 +324,7 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
             for i, r in zip(fused_ix, part):
                 out[i] = r
         for i in plain_ix:
-            r = _plain_scan(targets, all_bases[i], layout)
+            r = _bounded_scan(targets, all_bases[i], layout)
             if host:
                 h = HostResult(len(targets), all_bases[i])
                 for dst, src in zip(h.t, (r.zchi2, r.zcoeff, r.penalty)):
@@ -306,6 +337,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     from .device import StatusWord
     st = StatusWord()
     bounds = _chunk_bounds(len(targets), chunk)
+    # the last targets that fill no block, whatever chunk they fall into
+    few0 = len(targets) - few_tail(len(targets))
     main = torch.cuda.current_stream()
     # consecutive chunks alternate between two compute streams, so that a
     # chunk's packing, y GEMMs and first scan launch need not wait for the
@@ -313,7 +346,7 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     # chunk's last tile wave leaves idle (each chunk has its own outputs,
     # tile counters and scratch, allocated on its own stream)
     lanes = [main] if len(bounds) == 1 else [main, _lane_stream()]
-    if len(lanes) > 1:
+    if len(lanes) > 1 and few0 > 0:
         # what the chunks share is made on main first: the bases and their
         # INT8 digit planes for the y GEMM (cached on each basis)
         yv = _lib.YGEMM_VARIANTS[resolve_y(None, layout)]
@@ -338,11 +371,12 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
                 pack = _pack_cache.get(("chunk", layout.signature, i0, len(sub)), sub,
                                        lambda: _pack_overlapped(sub, layout, st, cs))
             tiles = None
-            if AUTOTUNE:
+            tail = max(0, i1 - max(i0, few0))
+            if AUTOTUNE and tail < len(sub):
                 from . import autotune
                 tiles = autotune.tiles_of(autotune.choice(pack, bases)
                                           or autotune.tune(pack, bases))
-            res, _ = run_fused(pack, bases, status=st, tiles=tiles)
+            res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=tail)
         keep.append((pack, res))
         if host:
             ev = torch.cuda.Event()
