@@ -329,6 +329,21 @@ int rr_zscan_pairs(const rr_pair_template* tmpl, const rr_pair_segment* segs /* 
                    int64_t npairs, double* chi2, double* coeff /* [npairs][nbasis] */,
                    double* penalty /* [npairs] or NULL */, int* status, rr_stream_t stream);
 
+/* The same pair scan in rounds through a workspace (16-byte aligned): the
+ * templates of a round's pairs are rebinned into it by the basis builder
+ * first, so the sums stream.  Same results bit for bit, several times
+ * faster.  rr_zscan_pairs_ws_bytes is the space for npairs pairs in one round
+ * (SIZE_MAX: bad arguments); with less -- the space of two pairs at least --
+ * the call takes as many rounds as it needs. */
+size_t rr_zscan_pairs_ws_bytes(const rr_pair_segment* segs, int nseg, int32_t nbasis,
+                               int64_t npairs);
+int rr_zscan_pairs_ws(const rr_pair_template* tmpl, const rr_pair_segment* segs /* host, <= 16 */,
+                      int nseg, const double* rows, const double* fwf, const double* wsum,
+                      int64_t npix_row, const int32_t* pair_target, const double* pair_z,
+                      int64_t npairs, double* chi2, double* coeff /* [npairs][nbasis] */,
+                      double* penalty /* [npairs] or NULL */, void* workspace,
+                      size_t workspace_bytes, int* status, rr_stream_t stream);
+
 /* ------------------------------------------------------------------------
  * Adjoint of the pair scan (differentiation of chi2(z), configuration
  * "Differentiation" of this engine; redrock refines z with the parabola of

@@ -130,6 +130,119 @@ static __device__ double transmission_inoue14(double z, double lobs) {
   return exp(dmul(-1.0, tau));
 }
 
+// The same transmission for many redshifts of one wavelength.  Every power of
+// the observed wavelength is kept between redshifts (they do not depend on
+// z), the powers of 1 + z come from the caller (they do not depend on the
+// wavelength), and the Lyman-series sums, whose terms depend on the
+// wavelength alone and whose lines are switched on from the longest one as
+// the rest wavelength falls (the table is in descending order), are extended
+// line by line as z grows and started again when it does not.  Every value is
+// the one transmission_inoue14 forms, by the same operations in the same
+// order.
+struct InoueZ {
+  double z, zp1;
+  double h;      // zp1^1.6 (z < 4.7) or zp1^3.4
+  double e, f;   // zp1^2 and zp1^2.3 (z < 2), or zp1^3 and zp1^3.3
+};
+
+static __device__ InoueZ inoue_z(double z) {
+  InoueZ c;
+  c.z = z;
+  c.zp1 = dadd(1.0, z);
+  if (z < 2.0) {
+    c.e = dmul(c.zp1, c.zp1);
+    c.f = pow(c.zp1, 2.3);
+  } else {
+    c.e = pow(c.zp1, 3.0);
+    c.f = pow(c.zp1, 3.3);
+  }
+  c.h = pow(c.zp1, z < 4.7 ? 1.6 : 3.4);
+  return c;
+}
+
+struct InoueWave {
+  double lobs;
+  double t_laf = 0.0, t_dla = 0.0;  // sums of the first nline lines
+  int nline = 0;
+  // powers of lobs and of lobs / kLamL, formed when first used (none is
+  // negative; -1: not yet)
+  double p12 = -1.0, p37 = -1.0, p55 = -1.0, p3 = -1.0;
+  double r_m03 = -1.0, r12 = -1.0, r21 = -1.0, r3 = -1.0, r37 = -1.0, r55 = -1.0;
+};
+
+static __device__ __noinline__ double igm_pow(double x, double e) { return pow(x, e); }
+__device__ __forceinline__ double kept_pow(double& v, double x, double e) {
+  if (v < 0) v = igm_pow(x, e);
+  return v;
+}
+
+__device__ __forceinline__ double transmission_inoue14(const InoueZ& zc, InoueWave& w) {
+  const double lobs = w.lobs;
+  const double lrest = ddiv(lobs, zc.zp1);
+  if (w.nline > 0 && !(lrest < c_inoue_lam[w.nline - 1])) {
+    w.nline = 0;
+    w.t_laf = 0.0;
+    w.t_dla = 0.0;
+  }
+  while (w.nline < RR_INOUE14_NLINES && lrest < c_inoue_lam[w.nline]) {
+    const int j = w.nline++;
+    const double l2 = c_inoue_lam[j];
+    double term;
+    if (lobs < dmul(l2, dadd(1.0, 1.2))) {
+      term = dmul(c_inoue_laf[j][0], kept_pow(w.p12, lobs, 1.2));
+    } else if (lobs < dmul(l2, dadd(1.0, 4.7))) {
+      term = dmul(c_inoue_laf[j][1], kept_pow(w.p37, lobs, 3.7));
+    } else {
+      term = dmul(c_inoue_laf[j][2], kept_pow(w.p55, lobs, 5.5));
+    }
+    w.t_laf = dadd(w.t_laf, term);
+    if (lobs < dmul(l2, dadd(1.0, 2.0)))
+      term = dmul(c_inoue_dla[j][0], dmul(lobs, lobs));
+    else
+      term = dmul(c_inoue_dla[j][1], kept_pow(w.p3, lobs, 3.0));
+    w.t_dla = dadd(w.t_dla, term);
+  }
+  double t_lcdla = 0.0, t_lclaf = 0.0;
+  if (lobs < dmul(kLamL, zc.zp1)) {
+    const double r = ddiv(lobs, kLamL);
+    const double r_m03 = kept_pow(w.r_m03, r, -3e-1);
+    if (zc.z < 2.0) {
+      t_lcdla = dsub(dsub(dmul(0.2113, zc.e), dmul(dmul(0.07661, zc.f), r_m03)),
+                     dmul(0.1347, dmul(r, r)));
+    } else if (lobs >= dmul(kLamL, dadd(1.0, 2.0))) {
+      t_lcdla = dsub(dsub(dmul(0.04696, zc.e), dmul(dmul(0.01779, zc.f), r_m03)),
+                     dmul(0.02916, kept_pow(w.r3, r, 3.0)));
+    } else {
+      t_lcdla = dsub(dsub(dsub(dadd(0.6340, dmul(0.04696, zc.e)),
+                               dmul(dmul(0.01779, zc.f), r_m03)),
+                          dmul(0.1347, dmul(r, r))),
+                     dmul(0.2905, r_m03));
+    }
+    const double i21 = kept_pow(w.r21, r, 2.1);
+    if (zc.z < 4.7) {
+      if (lobs >= dmul(kLamL, dadd(1.0, 1.2)))
+        t_lclaf = dmul(2.545e-2, dsub(dmul(zc.h, i21), kept_pow(w.r37, r, 3.7)));
+      else
+        t_lclaf = dsub(dadd(dmul(dmul(2.545e-2, zc.h), i21),
+                            dmul(0.3248, kept_pow(w.r12, r, 1.2))),
+                       dmul(0.2496, i21));
+    } else if (lobs > dmul(kLamL, dadd(1.0, 4.7))) {
+      t_lclaf = dmul(5.221e-4, dsub(dmul(zc.h, i21), kept_pow(w.r55, r, 5.5)));
+    } else if (lobs >= dmul(kLamL, dadd(1.0, 1.2)) && lobs < dmul(kLamL, dadd(1.0, 4.7))) {
+      t_lclaf = dsub(dadd(dmul(dmul(5.221e-4, zc.h), i21), dmul(0.2182, i21)),
+                     dmul(2.545e-2, kept_pow(w.r37, r, 3.7)));
+    } else if (lobs < dmul(kLamL, dadd(1.0, 1.2))) {
+      t_lclaf = dsub(dadd(dmul(dmul(5.221e-4, zc.h), i21),
+                          dmul(0.3248, kept_pow(w.r12, r, 1.2))),
+                     dmul(3.140e-2, i21));
+    }
+  }
+  const double tau_ls = dadd(w.t_laf, w.t_dla);
+  const double tau_lc = dadd(t_lclaf, t_lcdla);
+  const double tau = dadd(dadd(tau_lc, tau_ls), 0.0);
+  return exp(dmul(-1.0, tau));
+}
+
 // Calura et al. (2012) / Kamble et al. (2020) effective optical depth of
 // the Lyman series lines (constants.py:16-37, igm.py:321-364).
 static __device__ double transmission_calura_kamble(int model, double z, double lobs) {
@@ -221,11 +334,10 @@ constexpr int kMaxRebinBasis = 16;
 // three dependent loads on the (usually uniform) template grids; a binary
 // search over what is left covers uneven grids.  Every comparison is the
 // exactly rounded x[j] (1+z) <= e, so the result is the binary search's.
-__device__ __forceinline__ int64_t first_above(const double* __restrict__ x, int64_t nx,
-                                               double zp1, double e) {
+// t is the guess (any value gives the same answer).
+__device__ __forceinline__ int64_t first_above_near(const double* __restrict__ x, int64_t nx,
+                                                    double zp1, double e, double t) {
   int64_t lo = 0, hi = nx;  // the answer lies in [lo, hi]
-  const double x0 = x[0];
-  const double t = (e / zp1 - x0) / (x[nx - 1] - x0) * (double)(nx - 1);
   if (t > 0.0 && t < (double)(nx - 1)) {
     const int64_t g = (int64_t)t;
     if (dmul(x[g], zp1) <= e) {
@@ -253,6 +365,13 @@ __device__ __forceinline__ int64_t first_above(const double* __restrict__ x, int
     if (dmul(x[mid], zp1) <= e) lo = mid + 1; else hi = mid;
   }
   return lo;
+}
+
+__device__ __forceinline__ int64_t first_above(const double* __restrict__ x, int64_t nx,
+                                               double zp1, double e) {
+  const double x0 = x[0];
+  return first_above_near(x, nx, zp1, e,
+                          (e / zp1 - x0) / (x[nx - 1] - x0) * (double)(nx - 1));
 }
 
 template <bool DZ = false>
@@ -318,6 +437,116 @@ __device__ __forceinline__ bool rebin_bin_strided(const double* __restrict__ x, 
   if (DZ)
     for (int b = 0; b < nb; ++b)
       dres[b] = (res[b] - (e_hi * yhi_e[b] - e_lo * ylo_e[b]) / width) / zp1;
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// the same rebin with shared, exactly corrected divisions
+// ---------------------------------------------------------------------------
+// RN(a / b) from r = RN(1 / b) by Markstein's method (IBM J. Res. Dev. 34,
+// 1990): q0 = a r lies within 1.5 ulp, one residual step makes it faithful,
+// and a residual step from a faithful quotient with the correctly rounded
+// reciprocal rounds correctly.  Five operations per quotient and one
+// reciprocal per divisor, where the bases of a bin share their divisors.
+// For a and b well inside the exponent range (div_range, div_range_b); bins
+// with others take rebin_bin_strided.  (A zero a gives +0 where the division
+// may give -0: the sums below start from +0, so no result shows it.)
+__device__ __forceinline__ double div_near(double a, double b, double r) {
+  double q = __dmul_rn(a, r);
+  q = __fma_rn(__fma_rn(-q, b, a), r, q);
+  return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+// |a| in 2^-511 .. 2^512, or 0
+__device__ __forceinline__ bool div_range(double a) {
+  const unsigned hi = (unsigned)__double2hiint(a);
+  return ((hi & 0x7fffffffu) - 0x20000000u < 0x40000000u) |
+         (((hi << 1) | (unsigned)__double2loint(a)) == 0u);
+}
+// b in 2^-63 .. 2^64, positive
+__device__ __forceinline__ bool div_range_b(double b) {
+  return (unsigned)__double2hiint(b) - 0x3c000000u < 0x08000000u;
+}
+
+// One bin for NB bases in registers: rebin_bin_strided's operations in its
+// order, each sample read once.  j is first_above(e_lo).  Returns false
+// when the bin falls outside the input range; exact is false when a division
+// was out of div_near's range and res is not to be used.
+template <int NB>
+__device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int64_t nx,
+                                              const double* __restrict__ y, int64_t ystride,
+                                              double zp1, double e_lo, double e_hi, int64_t j,
+                                              double (&res)[NB], bool& exact) {
+  if (j < 1 || j >= nx) return false;
+  double xj = dmul(x[j], zp1);
+  const double xjm1 = dmul(x[j - 1], zp1);
+  double yc[NB], yn[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) yc[b] = y[(int64_t)b * ystride + j];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) yn[b] = y[(int64_t)b * ystride + j - 1];
+  double dx = dsub(xj, xjm1);
+  double r = __drcp_rn(dx);
+  bool ok = div_range_b(dx);
+  if (xj < e_hi) {
+    // lower edge to the first sample inside the bin
+    double t = dsub(e_lo, xjm1);
+    const double h = dsub(xj, e_lo);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const double a = dmul(t, dsub(yc[b], yn[b]));
+      ok = ok & div_range(a);
+      const double yedge = dadd(yn[b], div_near(a, dx, r));
+      res[b] = dadd(0.0, dmul(dmul(0.5, dadd(yc[b], yedge)), h));
+    }
+    // interior samples
+    while (true) {
+      if (j + 1 >= nx) return false;
+      const double xn = dmul(x[j + 1], zp1);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) yn[b] = y[(int64_t)b * ystride + j + 1];
+      dx = dsub(xn, xj);
+      if (!(xn < e_hi)) break;
+      ++j;
+      xj = xn;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        res[b] = dadd(res[b], dmul(dmul(0.5, dadd(yn[b], yc[b])), dx));
+        yc[b] = yn[b];
+      }
+    }
+    // upper edge
+    t = dsub(e_hi, xj);
+    r = __drcp_rn(dx);
+    ok = ok & div_range_b(dx);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const double a = dmul(t, dsub(yn[b], yc[b]));
+      ok = ok & div_range(a);
+      const double yedge = dadd(yc[b], div_near(a, dx, r));
+      res[b] = dadd(res[b], dmul(dmul(0.5, dadd(yedge, yc[b])), t));
+    }
+  } else {
+    // the samples span the whole bin
+    const double tl = dsub(e_lo, xj), th = dsub(e_hi, xj), w = dsub(e_hi, e_lo);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const double slope = dsub(yc[b], yn[b]);
+      const double al = dmul(tl, slope), ah = dmul(th, slope);
+      ok = ok & div_range(al) & div_range(ah);
+      const double ylo = dadd(yc[b], div_near(al, dx, r));
+      const double yhi = dadd(yc[b], div_near(ah, dx, r));
+      res[b] = dadd(0.0, dmul(dmul(0.5, dadd(ylo, yhi)), w));
+    }
+  }
+  const double width = dsub(e_hi, e_lo);
+  r = __drcp_rn(width);
+  ok = ok & div_range_b(width);
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    ok = ok & div_range(res[b]);
+    res[b] = div_near(res[b], width, r);
+  }
+  exact = ok;
   return true;
 }
 

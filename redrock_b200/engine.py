@@ -697,6 +697,25 @@ def pair_ranges_ok(src, layout, z):
     return ok
 
 
+# workspace of a pair scan: the rebinned templates of one round of pairs
+# (642 KB per pair at 10 bases on DESI grids)
+PAIR_WS_BYTES = 1 << 30
+
+
+def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream):
+    """rr_zscan_pairs_ws over device pairs, in rounds of PAIR_WS_BYTES."""
+    L = _lib.lib()
+    nseg = len(rowpack.segments)
+    need = int(L.rr_zscan_pairs_ws_bytes(segs, nseg, tm.nbasis, n + n % 2))
+    two = int(L.rr_zscan_pairs_ws_bytes(segs, nseg, tm.nbasis, 2))
+    ws = torch.empty(min(need, max(two, PAIR_WS_BYTES)), dtype=torch.uint8, device=chi2.device)
+    rc = L.rr_zscan_pairs_ws(ctypes.byref(tm), segs, nseg, ptr(rowpack.rows), ptr(rowpack.fwf),
+                             ptr(rowpack.wsum), rowpack.npix_row, ptr(pair_target), ptr(pair_z), n,
+                             ptr(chi2), ptr(coeff), ptr(pen), ptr(ws), ws.numel(), status.ptr,
+                             stream_handle(stream))
+    _lib.check(rc, "rr_zscan_pairs_ws")
+
+
 def run_pairs(rowpack, src, pair_target, pair_z, stream=None, status=None, bounds=None):
     """chi2 (n,), coeff (n, nbasis), penalty (n,) device tensors for the
     pairs (target index into the packed targets, redshift).  ``bounds``:
@@ -723,10 +742,7 @@ def run_pairs(rowpack, src, pair_target, pair_z, stream=None, status=None, bound
                            None if hb is None else hb.ctypes.data_as(ctypes.c_void_p))
     segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
     st = status or StatusWord(dev)
-    rc = L.rr_zscan_pairs(ctypes.byref(tm), segs, len(rowpack.segments), ptr(rowpack.rows),
-                          ptr(rowpack.fwf), ptr(rowpack.wsum), rowpack.npix_row, ptr(dt), ptr(dz),
-                          n, ptr(chi2), ptr(coeff), ptr(pen), st.ptr, stream_handle(stream))
-    _lib.check(rc, "rr_zscan_pairs")
+    _pair_scan(rowpack, tm, segs, dt, dz, n, chi2, coeff, pen, st, stream)
     if status is None:
         torch.cuda.current_stream().synchronize()
         st.check("rr_zscan_pairs")
@@ -750,11 +766,7 @@ def run_pairs_device(rowpack, src, pair_target, pair_z, status, stream=None):
     tm = _lib.PairTemplate(ptr(src.x), src.nx, ptr(src.y), nb, src.igm, src.method, 0,
                            ptr(prior), ptr(src.oii_dev))
     segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
-    rc = L.rr_zscan_pairs(ctypes.byref(tm), segs, len(rowpack.segments), ptr(rowpack.rows),
-                          ptr(rowpack.fwf), ptr(rowpack.wsum), rowpack.npix_row, ptr(pair_target),
-                          ptr(pair_z), n, ptr(chi2), ptr(coeff), ptr(pen), status.ptr,
-                          stream_handle(stream))
-    _lib.check(rc, "rr_zscan_pairs")
+    _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream)
     return chi2, coeff, pen
 
 
