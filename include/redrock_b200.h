@@ -101,6 +101,11 @@ const char* rr_status_string(int status);
 /* last cudaError_t seen by a call of this library on this thread */
 int rr_last_cuda_error(void);
 
+/* Host helper: the n host arrays src[i] of bytes[i] bytes end to end into dst
+ * (dst_bytes long), by several threads when large.  Synchronous; no CUDA. */
+int rr_host_gather(const void* const* src, const int64_t* bytes, int64_t n, void* dst,
+                   int64_t dst_bytes);
+
 /* ------------------------------------------------------------------------
  * Trapezoidal rebinning of y(x (1+z)) onto bin edges, for every z and basis.
  *   x[nx] increasing; y[nbasis][nx]; edges[nbin+1]; z[nz]

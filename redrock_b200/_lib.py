@@ -122,6 +122,7 @@ _SIGNATURES = {
     "rr_zscan_fused_opt": (c_int, [ctypes.POINTER(ScanTargets), ctypes.POINTER(ScanTemplate),
                                    c_int, c_void_p, ctypes.POINTER(ScanOptions), c_void_p,
                                    c_void_p]),
+    "rr_host_gather": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int64]),
     "rr_few_rows_doubles": (c_int64, [ctypes.POINTER(ScanTargets)]),
     "rr_pack_few": (c_int, [ctypes.POINTER(ScanTargets), c_int64, c_int32, c_void_p, c_void_p]),
     "rr_zscan_few": (c_int, [ctypes.POINTER(ScanTargets), c_int64, c_int32, c_void_p,

@@ -31,6 +31,7 @@ import torch
 
 from . import _lib
 from .device import StatusWord, device, ptr, stream_handle, struct_bytes, to_device
+from .engine import _concat
 
 
 def _groups(target):
@@ -77,9 +78,14 @@ def coadd_targets(targets, cache_Rcsr=False, cosmics_nsig=0.):
     dg = to_device(struct_bytes(descs), torch.uint8)
     ded = to_device(np.asarray(exp_data, dtype=np.int64), torch.int64)
     dep = to_device(np.asarray(exp_pix, dtype=np.int64), torch.int64)
-    drd = to_device(np.concatenate(rdata))
-    div = to_device(np.concatenate(ivar))
-    dfl = to_device(np.concatenate(flux))
+    # gathered straight into pinned memory for the upload
+    pinned = {}
+
+    def up(name, parts):
+        a = _concat(parts, np.float64, pinned, name)
+        t = pinned.get(name)
+        return to_device(a) if t is None else t.to(dev, non_blocking=True)
+    drd, div, dfl = up("rdata", rdata), up("ivar", ivar), up("flux", flux)
     ord_ = torch.empty(max(out_data, 1), dtype=torch.float64, device=dev)
     oiv = torch.empty(max(out_pix, 1), dtype=torch.float64, device=dev)
     ofl = torch.empty(max(out_pix, 1), dtype=torch.float64, device=dev)

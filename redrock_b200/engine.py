@@ -341,13 +341,20 @@ def _concat(parts, dtype, pinned=None, name=None):
     """Concatenate 1-D arrays; into a pinned host tensor (kept in
     pinned[name]) when pinned is given, the result is >= 1 MB and a GPU is
     present."""
+    dt = np.dtype(dtype)
     n = sum(p.size for p in parts)
-    if (pinned is not None and n * np.dtype(dtype).itemsize >= (1 << 20)
-            and torch.cuda.is_available()):
+    if pinned is not None and n * dt.itemsize >= (1 << 20) and torch.cuda.is_available():
         t = torch.empty(n, dtype=torch.from_numpy(np.empty(0, dtype=dtype)).dtype,
                         pin_memory=True)
         pinned[name] = t
         out = t.numpy()
+        if all(p.dtype == dt and p.flags.c_contiguous for p in parts):
+            src = np.array([p.ctypes.data for p in parts], dtype=np.uintp)
+            size = np.array([p.nbytes for p in parts], dtype=np.int64)
+            rc = _lib.lib().rr_host_gather(src.ctypes.data, size.ctypes.data, len(parts),
+                                           out.ctypes.data, out.nbytes)
+            _lib.check(rc, "rr_host_gather")
+            return out
     else:
         out = np.empty(n, dtype=dtype)
     i = 0
