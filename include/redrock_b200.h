@@ -378,6 +378,17 @@ int rr_zscan_pairs_grad(const rr_pair_template* tmpl, const rr_pair_segment* seg
                         double* dchi2_dflux, double* dpenalty_dz, int* status,
                         rr_stream_t stream);
 
+/* rr_zscan_pairs_grad through a workspace, as rr_zscan_pairs_ws. */
+size_t rr_zscan_pairs_grad_ws_bytes(const rr_pair_segment* segs, int nseg, int32_t nbasis,
+                                    int64_t npairs);
+int rr_zscan_pairs_grad_ws(const rr_pair_template* tmpl, const rr_pair_segment* segs, int nseg,
+                           const double* rows, const double* sw, const double* fwf,
+                           const double* wsum, int64_t npix_row, const int32_t* pair_target,
+                           const double* pair_z, int64_t npairs, double* chi2, double* coeff,
+                           double* penalty, double* dchi2_dz, double* d2chi2_dz2,
+                           double* dchi2_dflux, double* dpenalty_dz, void* workspace,
+                           size_t workspace_bytes, int* status, rr_stream_t stream);
+
 /* ------------------------------------------------------------------------
  * fitz candidates on the device: replaces the host steps of redrock's fitz
  * between the coarse scan and the fine-grid evaluations --

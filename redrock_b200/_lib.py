@@ -144,6 +144,13 @@ _SIGNATURES = {
                                   c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                                   c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
                                   c_void_p, c_void_p]),
+    "rr_zscan_pairs_grad_ws_bytes": (c_size_t, [ctypes.POINTER(PairSegment), c_int, c_int32,
+                                                c_int64]),
+    "rr_zscan_pairs_grad_ws": (c_int, [ctypes.POINTER(PairTemplate), ctypes.POINTER(PairSegment),
+                                       c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                       c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
+                                       c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
+                                       c_void_p, c_void_p]),
     "rr_fitz_candidates": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int32,
                                    c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p]),

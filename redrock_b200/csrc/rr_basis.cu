@@ -94,15 +94,24 @@ static __device__ __noinline__ double transmission_plain(int model, double z, do
   return transmission(model, z, lobs);
 }
 
-template <int NB>
+template <int NB, bool DZ>
 __device__ __noinline__ bool rebin_bin_general(const double* __restrict__ x, int64_t nx,
                                                const double* __restrict__ y, double zp1,
-                                               double e_lo, double e_hi, double (&res)[NB]) {
-  double v[kMaxRebinBasis];
-  if (!rebin_bin(x, nx, y, NB, zp1, e_lo, e_hi, v)) return false;
+                                               double e_lo, double e_hi, double (&res)[NB],
+                                               double (&dres)[DZ ? NB : 1]) {
+  double v[kMaxRebinBasis], dv[DZ ? kMaxRebinBasis : 1];
+  if (!rebin_bin_strided<DZ>(x, nx, y, nx, NB, zp1, e_lo, e_hi, v, dv)) return false;
 #pragma unroll
   for (int b = 0; b < NB; ++b) res[b] = v[b];
+  if (DZ)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) dres[b] = dv[b];
   return true;
+}
+
+// d/dz of the Inoue14 factor t (the other models' is 0 between their steps)
+static __device__ __noinline__ double transmission_slope(double t, double z, double lobs) {
+  return -t * dtau_lc_dz_inoue14(z, lobs);
 }
 
 // The builder for basis rows of NB values (rounded up to even), all grids in
@@ -132,14 +141,15 @@ struct BuildParams {
   int ngrid;
   int igm_model;
   double* basis;
+  double* dbasis;  // dT/dz in the same layout (DZ)
   int64_t pix_stride;
   int* bad;       // per redshift: 1 where a bin fell outside the template, or NULL
   int* status;    // RR_ERANGE there, or NULL
 };
 
-// INOUE: the Inoue14 factor; else the other models, or none
-template <int NB, bool INOUE>
-__global__ void __launch_bounds__(kBuildThreads, 4) build_basis_kernel(
+// INOUE: the Inoue14 factor; else the other models, or none.  DZ: dT/dz too.
+template <int NB, bool INOUE, bool DZ>
+__global__ void __launch_bounds__(kBuildThreads, (DZ ? 3 : 4)) build_basis_kernel(
     const __grid_constant__ BuildParams p) {
   constexpr int S = (NB + 1) & ~1;
   constexpr int kZ = build_z(INOUE);
@@ -182,17 +192,21 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_basis_kernel(
   double* row = stage + threadIdx.x * S;
   for (int k = 0; k < nz; ++k) {
     const int64_t iz = z0 + k;
-    double res[NB];
+    double res[NB], dres[DZ ? NB : 1];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) res[b] = 0.0;
+    for (int b = 0; b < NB; ++b) {
+      res[b] = 0.0;
+      if (DZ) dres[b] = 0.0;
+    }
     if (real) {
       const double zz = p.z[iz];
       const double zp1 = dadd(1.0, zz);
       const int64_t j =
           first_above_near(p.x, p.nx, zp1, e_lo, (e_lo * __drcp_rn(zp1) - x0) * per_x);
       bool exact = true;
-      bool in = rebin_bin_reg<NB>(p.x, p.nx, p.y, p.nx, zp1, e_lo, e_hi, j, res, exact);
-      if (in && !exact) in = rebin_bin_general<NB>(p.x, p.nx, p.y, zp1, e_lo, e_hi, res);
+      bool in = rebin_bin_reg<NB, DZ>(p.x, p.nx, p.y, p.nx, zp1, e_lo, e_hi, j, res, exact, dres);
+      if (in && !exact)
+        in = rebin_bin_general<NB, DZ>(p.x, p.nx, p.y, zp1, e_lo, e_hi, res, dres);
       if (!in) {
         set_status(p.status, RR_ERANGE);
         if (p.bad) p.bad[iz] = 1;
@@ -201,23 +215,31 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_basis_kernel(
       } else if (s_igm[k]) {
         const double t = INOUE ? transmission_inoue14(zc[INOUE ? k : 0], wv)
                                : transmission_plain(p.igm_model, zz, wv.lobs);
+        if (DZ) {
+          const double dt = INOUE ? transmission_slope(t, zz, wv.lobs) : 0.0;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) dres[b] = dres[b] * t + res[b] * dt;
+        }
 #pragma unroll
         for (int b = 0; b < NB; ++b) res[b] = dmul(res[b], t);
       }
     }
 #pragma unroll
-    for (int b = 0; b < NB; ++b) row[b] = res[b];
-    if (NB & 1) row[S - 1] = 0.0;
-    __syncwarp();
-    const double2* src = reinterpret_cast<const double2*>(stage + warp * 32 * S);
-    double2* dst = reinterpret_cast<double2*>(
-        p.basis + (iz * p.pix_stride + gd.pix_offset - kHalfBand + first) * S);
+    for (int d = 0; d < (DZ ? 2 : 1); ++d) {
 #pragma unroll
-    for (int c = 0; c < S / 2; ++c) {
-      const int q = c * 32 + lane;
-      if (q < nrow * (S / 2)) dst[q] = src[q];
+      for (int b = 0; b < NB; ++b) row[b] = d ? dres[DZ ? b : 0] : res[b];
+      if (NB & 1) row[S - 1] = 0.0;
+      __syncwarp();
+      const double2* src = reinterpret_cast<const double2*>(stage + warp * 32 * S);
+      double2* dst = reinterpret_cast<double2*>(
+          (d ? p.dbasis : p.basis) + (iz * p.pix_stride + gd.pix_offset - kHalfBand + first) * S);
+#pragma unroll
+      for (int c = 0; c < S / 2; ++c) {
+        const int q = c * 32 + lane;
+        if (q < nrow * (S / 2)) dst[q] = src[q];
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -228,19 +250,24 @@ static int launch_build(const BuildParams& p, cudaStream_t stream) {
   const bool inoue = igm && p.igm_model == RR_IGM_INOUE14;
   const int kz = build_z(inoue);
   dim3 grid((unsigned)p.first[p.ngrid], (unsigned)((p.nz + kz - 1) / kz));
-  if (inoue)
-    build_basis_kernel<NB, true><<<grid, kBuildThreads, 0, stream>>>(p);
+  if (p.dbasis && inoue)
+    build_basis_kernel<NB, true, true><<<grid, kBuildThreads, 0, stream>>>(p);
+  else if (p.dbasis)
+    build_basis_kernel<NB, false, true><<<grid, kBuildThreads, 0, stream>>>(p);
+  else if (inoue)
+    build_basis_kernel<NB, true, false><<<grid, kBuildThreads, 0, stream>>>(p);
   else
-    build_basis_kernel<NB, false><<<grid, kBuildThreads, 0, stream>>>(p);
+    build_basis_kernel<NB, false, false><<<grid, kBuildThreads, 0, stream>>>(p);
   RR_CHECK_LAUNCH();
   return RR_OK;
 }
 
 int build_basis_rows(const double* x, int64_t nx, const double* y, int nbasis, const double* z,
                      int64_t nz, const BuildGrid* grids, int ngrid, int igm_model,
-                     int64_t pix_stride, double* basis, int* bad, int* status,
+                     int64_t pix_stride, double* basis, double* dbasis, int* bad, int* status,
                      cudaStream_t stream) {
   BuildParams p{};
+  p.dbasis = dbasis;
   p.x = x;
   p.nx = nx;
   p.y = y;
@@ -350,7 +377,7 @@ extern "C" int rr_build_basis(const double* x, int64_t nx, const double* y, int6
                           gd.apply_igm && igm_model != RR_IGM_NONE};
       }
       rc = build_basis_rows(x, nx, y, (int)nbasis, z, nz, bg, n, igm_model, pix_stride, basis,
-                            nullptr, status, (cudaStream_t)stream);
+                            nullptr, nullptr, status, (cudaStream_t)stream);
       if (rc) return rc;
     }
     return RR_OK;

@@ -21,10 +21,10 @@ struct BuildGrid {
 
 // Basis rows of nbasis (<= 10) values rounded up to even, 16-byte aligned, of
 // nz redshifts on the given grids; the tables of basis_tables are uploaded.
-// bad[iz] = 1 and status RR_ERANGE where a bin falls outside the template.
+// dbasis (or NULL) gets dT/dz in the same layout; bad[iz] = 1 and status RR_ERANGE where a bin falls outside the template.
 int build_basis_rows(const double* x, int64_t nx, const double* y, int nbasis, const double* z,
                      int64_t nz, const BuildGrid* grids, int ngrid, int igm_model,
-                     int64_t pix_stride, double* basis, int* bad, int* status,
+                     int64_t pix_stride, double* basis, double* dbasis, int* bad, int* status,
                      cudaStream_t stream);
 int basis_tables(cudaStream_t stream);
 

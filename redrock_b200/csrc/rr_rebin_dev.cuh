@@ -470,12 +470,14 @@ __device__ __forceinline__ bool div_range_b(double b) {
 // One bin for NB bases in registers: rebin_bin_strided's operations in its
 // order, each sample read once.  j is first_above(e_lo).  Returns false
 // when the bin falls outside the input range; exact is false when a division
-// was out of div_near's range and res is not to be used.
-template <int NB>
+// was out of div_near's range and res is not to be used.  With DZ, dres gets
+// dT/dz from the edge values, as in rebin_bin_strided (to a rounding or two).
+template <int NB, bool DZ = false>
 __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int64_t nx,
                                               const double* __restrict__ y, int64_t ystride,
                                               double zp1, double e_lo, double e_hi, int64_t j,
-                                              double (&res)[NB], bool& exact) {
+                                              double (&res)[NB], bool& exact,
+                                              double (&dres)[DZ ? NB : 1]) {
   if (j < 1 || j >= nx) return false;
   double xj = dmul(x[j], zp1);
   const double xjm1 = dmul(x[j - 1], zp1);
@@ -496,6 +498,7 @@ __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int6
       const double a = dmul(t, dsub(yc[b], yn[b]));
       ok = ok & div_range(a);
       const double yedge = dadd(yn[b], div_near(a, dx, r));
+      if (DZ) dres[b] = -e_lo * yedge;
       res[b] = dadd(0.0, dmul(dmul(0.5, dadd(yc[b], yedge)), h));
     }
     // interior samples
@@ -523,6 +526,7 @@ __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int6
       const double a = dmul(t, dsub(yn[b], yc[b]));
       ok = ok & div_range(a);
       const double yedge = dadd(yc[b], div_near(a, dx, r));
+      if (DZ) dres[b] = fma(e_hi, yedge, dres[b]);
       res[b] = dadd(res[b], dmul(dmul(0.5, dadd(yedge, yc[b])), t));
     }
   } else {
@@ -535,6 +539,7 @@ __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int6
       ok = ok & div_range(al) & div_range(ah);
       const double ylo = dadd(yc[b], div_near(al, dx, r));
       const double yhi = dadd(yc[b], div_near(ah, dx, r));
+      if (DZ) dres[b] = fma(e_hi, yhi, -e_lo * ylo);
       res[b] = dadd(0.0, dmul(dmul(0.5, dadd(ylo, yhi)), w));
     }
   }
@@ -545,6 +550,7 @@ __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int6
   for (int b = 0; b < NB; ++b) {
     ok = ok & div_range(res[b]);
     res[b] = div_near(res[b], width, r);
+    if (DZ) dres[b] = (res[b] - dres[b] * r) / zp1;
   }
   exact = ok;
   return true;

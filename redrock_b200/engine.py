@@ -709,13 +709,18 @@ def pair_ranges_ok(src, layout, z):
 PAIR_WS_BYTES = 1 << 30
 
 
+def _pair_ws(nbytes, segs, nbasis, n, dev):
+    """Workspace of n pairs, at most PAIR_WS_BYTES (but two pairs)."""
+    need = int(nbytes(segs, len(segs), nbasis, n + n % 2))
+    two = int(nbytes(segs, len(segs), nbasis, 2))
+    return torch.empty(min(need, max(two, PAIR_WS_BYTES)), dtype=torch.uint8, device=dev)
+
+
 def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream):
     """rr_zscan_pairs_ws over device pairs, in rounds of PAIR_WS_BYTES."""
     L = _lib.lib()
     nseg = len(rowpack.segments)
-    need = int(L.rr_zscan_pairs_ws_bytes(segs, nseg, tm.nbasis, n + n % 2))
-    two = int(L.rr_zscan_pairs_ws_bytes(segs, nseg, tm.nbasis, 2))
-    ws = torch.empty(min(need, max(two, PAIR_WS_BYTES)), dtype=torch.uint8, device=chi2.device)
+    ws = _pair_ws(L.rr_zscan_pairs_ws_bytes, segs, tm.nbasis, n, chi2.device)
     rc = L.rr_zscan_pairs_ws(ctypes.byref(tm), segs, nseg, ptr(rowpack.rows), ptr(rowpack.fwf),
                              ptr(rowpack.wsum), rowpack.npix_row, ptr(pair_target), ptr(pair_z), n,
                              ptr(chi2), ptr(coeff), ptr(pen), ptr(ws), ws.numel(), status.ptr,
@@ -828,11 +833,12 @@ def run_pairs_grad(rowpack, src, pair_target, pair_z, want_dflux=False, stream=N
                            ptr(oii))
     segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
     st = status or StatusWord(dev)
-    rc = L.rr_zscan_pairs_grad(ctypes.byref(tm), segs, len(rowpack.segments), ptr(rowpack.rows),
-                               ptr(rowpack.sw), ptr(rowpack.fwf), ptr(rowpack.wsum),
-                               rowpack.npix_row, ptr(dt), ptr(dz), n, ptr(chi2), ptr(coeff),
-                               ptr(pen), ptr(g), ptr(h), ptr(df), ptr(dp), st.ptr,
-                               stream_handle(stream))
+    ws = _pair_ws(L.rr_zscan_pairs_grad_ws_bytes, segs, nb, n, dev)
+    rc = L.rr_zscan_pairs_grad_ws(ctypes.byref(tm), segs, len(rowpack.segments),
+                                  ptr(rowpack.rows), ptr(rowpack.sw), ptr(rowpack.fwf),
+                                  ptr(rowpack.wsum), rowpack.npix_row, ptr(dt), ptr(dz), n,
+                                  ptr(chi2), ptr(coeff), ptr(pen), ptr(g), ptr(h), ptr(df),
+                                  ptr(dp), ptr(ws), ws.numel(), st.ptr, stream_handle(stream))
     _lib.check(rc, "rr_zscan_pairs_grad")
     if status is None:
         torch.cuda.current_stream().synchronize()
