@@ -26,16 +26,18 @@ namespace rr {
 #define RR_PIX 4
 #endif
 #ifndef RR_PIX_SMALL
-#define RR_PIX_SMALL RR_PIX
+#define RR_PIX_SMALL 8
 #endif
 
 constexpr int kQUnroll = RR_Q_UNROLL;
-// pixels per step of the pixel loop: RR_PIX for the instantiations whose
-// accumulators fill the register file (NB * ZT > 10), RR_PIX_SMALL for the
-// others
+// pixels per step of the pixel loop: RR_PIX_SMALL where the accumulators leave
+// registers for it (each basis row is then read for eight pixels: STAR at one
+// redshift per thread 11.4 -> 10.7 ms on 448 targets, QSO at one and two 65.0
+// -> 60.4 and 58.8 -> 56.1), else RR_PIX (with eight they spill: GALAXY 141 ->
+// 200 ms)
 template <int NB, int ZT>
 constexpr int pix_per_step() {
-  return NB * ZT > 10 ? RR_PIX : RR_PIX_SMALL;
+  return NB <= 5 && NB * ZT <= 8 ? RR_PIX_SMALL : RR_PIX;
 }
 constexpr int kWarps = RR_SCAN_WARPS;  // redshifts per tile (one per warp)
 constexpr int kThreads = kWarps * 32;
@@ -229,12 +231,20 @@ __device__ __forceinline__ bool sweep(const FusedParams& p, const rr_scan_templa
 #pragma unroll
             for (int b = 0; b + 1 < NB; b += 2) {
               const double2 tv = *reinterpret_cast<const double2*>(trow + b);
+              // back and forth over the pixels, so that every product
+              // shares a factor with the one before: three new 64-bit
+              // operands take a DFMA three register-file cycles, two the two
+              // of the FP64 pipe (registers only: 77 -> 90 % of its peak;
+              // here GALAXY 145.6 -> 141.3 ms and QSO 56.6 -> 55.0 ms on 448
+              // targets, the shared-memory reads now bounding the loop: 81 %
+              // of peak without its copies and barriers)
 #pragma unroll
-              for (int i = 0; i < kPix; ++i) {
-                if (k - i >= 0 && k - i < kBand) {
-                  tp[j][i][b] = fma(rk[i], tv.x, tp[j][i][b]);
-                  tp[j][i][b + 1] = fma(rk[i], tv.y, tp[j][i][b + 1]);
-                }
+              for (int i = 0; i < kPix; ++i)
+                if (k - i >= 0 && k - i < kBand) tp[j][i][b] = fma(rk[i], tv.x, tp[j][i][b]);
+#pragma unroll
+              for (int ii = 0; ii < kPix; ++ii) {
+                const int i = kPix - 1 - ii;
+                if (k - i >= 0 && k - i < kBand) tp[j][i][b + 1] = fma(rk[i], tv.y, tp[j][i][b + 1]);
               }
             }
             if (NB & 1) {
