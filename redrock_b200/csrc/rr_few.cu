@@ -4,8 +4,8 @@
 
 namespace rr {
 
-// lrows[i][step][k][q][lane] = rw of target first + i at pixel p0 + 3 lane + q
-// of the step, 0 past the segment's padded end.  Reads one 8-byte column of
+// lrows[i][step][k][q][g] = rw of target first + i at pixel p0 + 3 g + q of the
+// step, 0 past the segment's padded end.  Reads one 8-byte column of
 // the fused scan's lane-fastest rows per target (a 32-byte sector each for
 // one target, whole sectors from four targets on): 3 MB for a DESI target
 // against the 2 GB of basis the scan then reads.

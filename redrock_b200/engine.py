@@ -525,10 +525,10 @@ def _record(ev, stream):
 
 # the last targets of a batch that do not fill a 32-target block of the
 # fused scan go through the few-target kernel when there are at most this
-# many of them: with all seven templates a target costs it 1.65 ms, a block
-# of the fused scan about 17 ms however many of its lanes are used (GALAXY
-# 10.5, QSO 4.4, STAR 2.6, measured at 37 targets)
-FEW_MAX = 10
+# many of them: with all seven templates a target costs it 0.80 ms (GALAXY
+# 0.53, QSO 0.23, STAR 0.04), a block of the fused scan 16 to 18 ms however
+# many of its lanes are used (GALAXY 10.5, QSO 4.2 to 7.9, STAR 2.6)
+FEW_MAX = 20
 
 
 def few_tail(ntarget):
