@@ -439,9 +439,11 @@ static int zscan_fused(const rr_scan_targets* targets, const rr_scan_template* t
   typedef int (*group_fn)(bool, int, int, const rr_scan_targets*, const rr_scan_template*,
                           const int*, int, int*, int*, int*, bool, cudaStream_t);
   const group_fn fns[kNGroups] = {fused_group_0, fused_group_1, fused_group_2, fused_group_3};
-  for (int gi = 0; gi < 2 * kNGroups && !rc; ++gi) {
+  // the largest bases first: the small ones then fill their last tile wave
+  for (int i = 0; i < 2 * kNGroups && !rc; ++i) {
+    const int g = i / 2;
+    const int gi = i % 2 ? g : g + kNGroups;
     if (!ng[gi]) continue;
-    const int g = gi % kNGroups;
     rc = fns[g](gi >= kNGroups, zt[g], bgroup, targets, templates, group[gi], ng[gi],
                 tile_counter + 4 + gi, resweep, status, overlap, st);
     overlap = true;

@@ -516,6 +516,25 @@ def resolve_y(ygemm, layout):
     return v
 
 
+def y_in_scan(basis, ntarget):
+    """Whether y of a batch of ntarget targets against this basis is cheaper
+    summed inside the scan (FP64) than as a tensor-core GEMM of its own.
+    The GEMM takes rounds of one 128-target x 80-column tile per SM, each as
+    long as the pixels are (0.33 ms for 8064), however few tiles there are:
+    five STAR templates of 100 redshifts cost it 1.7 ms at any batch up to
+    1000 targets.  The scan sums y at 13 TFMA/s; ten bases leave it no
+    registers for y and pay about twice that (32 targets: GALAXY 11.4 ms with
+    the GEMM and 12.0 without, QSO 5.7 and 5.3, STAR 3.5 and 1.9; the QSO lines
+    cross between 64 and 96 targets, 10.2 / 10.0 and 13.0 / 13.2 ms)."""
+    L = _lib.lib()
+    kpad = int(L.rr_ygemm_kpad(basis.layout.pix_stride))
+    tiles = -(-basis.nz // (80 // basis.nbasis)) * -(-ntarget // 128)
+    gemm = -(-tiles // 148) * (kpad / 32) * 1.32e-6
+    lanes = round_up(max(ntarget, 1), _lib.LANES)
+    scan = lanes * basis.nz * basis.layout.pix_stride * basis.nbasis / 13.3e12
+    return scan * (2.3 if basis.nbasis > 5 else 1.0) < gemm
+
+
 def _record(ev, stream):
     if isinstance(stream, torch.cuda.Stream):
         ev.record(stream)
@@ -574,10 +593,13 @@ class FewRows:
 
 
 def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=None,
-              tiles=None, external_events=False, tail=None):
+              tiles=None, external_events=False, tail=None, ntarget=None):
     """One persistent launch over every (target, template, z).  ygemm:
-    None (DEFAULT_Y), "fp64", "int8x6", "int8x7", "bf16x3" or "tf32x3"; other than
-    "fp64", y is computed on the tensor cores first (YGemm).  kernel_events:
+    None (DEFAULT_Y, or "fp64" for the templates y_in_scan says), "fp64", "int8x6",
+    "int8x7", "bf16x3" or "tf32x3"; other than
+    "fp64", y is computed on the tensor cores first (YGemm).  ntarget: the size
+    of the whole batch when the pack is a chunk of it (y_in_scan's choice must
+    not depend on the chunks).  kernel_events:
     a list that gets a (start, end) CUDA event pair around the scan launches
     alone (timing).  tiles: redshifts per thread {nbasis: ZT} for the small
     bases (nbasis 4: 1-3, nbasis 5: 1-2; rr_scan_options) and optionally
@@ -608,17 +630,19 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
             rows = pack.rows.clone()
             rows[nfull:] = -1
         tgs = pack.scan_targets_struct(nblock, rows)
+        inside = [False] * len(bases)
+        if ygemm is None:
+            inside = [y_in_scan(b, ntarget or pack.ntarget) for b in bases]
         ygemm = resolve_y(ygemm, pack.layout)
-        yg = None if ygemm == "fp64" else YGemm(pack, ygemm, stream=stream, status=st,
-                                                nblock=nblock)
+        yg = None if ygemm == "fp64" or all(inside) else \
+            YGemm(pack, ygemm, stream=stream, status=st, nblock=nblock)
     for i0 in range(0, len(bases), _lib.MAX_TEMPLATES):
         sub = bases[i0:i0 + _lib.MAX_TEMPLATES]
         out = results[i0:i0 + _lib.MAX_TEMPLATES]
         if fused:
-            if yg is not None:
-                for b, r in zip(sub, out):
-                    # kept with the result so it outlives the launch
-                    r.y_ext = yg.y(b, stream=stream)
+            for b, r, ins in zip(sub, out, inside[i0:]):
+                # kept with the result so it outlives the launch
+                r.y_ext = yg.y(b, stream=stream) if yg is not None and not ins else None
             tms = _scan_templates(sub, out)
             arr = (_lib.ScanTemplate * len(tms))(*tms)
             if kernel_events is not None:

@@ -31,7 +31,7 @@ import torch
 from . import _lib
 from .device import to_device, to_numpy
 from .engine import (DeviceBasis, FewRows, GridLayout, IdCache, PlainTarget, ScanResult,
-                     TargetBatch, TargetPack, few_tail, resolve_y, run_fused, run_plain)
+                     TargetBatch, TargetPack, few_tail, resolve_y, run_fused, run_plain, y_in_scan)
 from .templates import oii_sums, solve_code, solve_code_of
 
 HUGE_CHI2 = 9999999.0
@@ -353,7 +353,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
         if yv in _lib.I8_VARIANTS:
             kpad = int(_lib.lib().rr_ygemm_kpad(layout.pix_stride))
             for b in bases:
-                b.i8_digits(kpad, variant=yv)
+                if not y_in_scan(b, len(targets)):
+                    b.i8_digits(kpad, variant=yv)
         ev0 = torch.cuda.Event()
         ev0.record(main)
         lanes[1].wait_event(ev0)
@@ -376,7 +377,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
                 from . import autotune
                 tiles = autotune.tiles_of(autotune.choice(pack, bases)
                                           or autotune.tune(pack, bases))
-            res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=tail)
+            res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=tail,
+                               ntarget=len(targets))
         keep.append((pack, res))
         if host:
             ev = torch.cuda.Event()

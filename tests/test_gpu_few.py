@@ -129,3 +129,30 @@ def test_bounded_scan_equals_plain_chain(method, nb, n):
     np.testing.assert_array_equal(co == 0, rc == 0)
     scale = np.maximum(np.abs(rc).max(axis=-1, keepdims=True), 1e-300)
     assert np.all(np.abs(co - rc) <= 1e-5 * scale)
+
+
+@pytest.mark.parametrize("n", [32, 70])
+def test_y_choice_per_template(n):
+    """The default y is the scan's own FP64 sum for the templates y_in_scan
+    names -- bit-identical to ygemm="fp64" there -- and the INT8 GEMM for the
+    others; the choice follows the whole batch, not the chunk."""
+    import torch
+    from redrock_b200 import targets as T, templates as TM, zscan
+    from redrock_b200.engine import TargetBatch, TargetPack, run_fused, y_in_scan
+    tg = T.from_synth(synth.make_targets(n, seed=87))
+    tset = synth.template_set()
+    sel = [tset[0], tset[2]]                       # GALAXY at full length, one STAR
+    dts = [TM.DistTemplate(TM.from_synth(t), synth.camera_grids()) for t in sel]
+    bases = [d.basis for d in dts]
+    assert not y_in_scan(bases[0], n) and y_in_scan(bases[1], n)
+    pack = TargetPack(TargetBatch(tg, dts[0].layout).to_device())
+    tail = n % 32
+    got, st = run_fused(pack, bases, tail=tail)
+    ref, st2 = run_fused(pack, bases, ygemm="fp64", tail=tail)
+    st.check("mixed")
+    st2.check("fp64")
+    assert torch.equal(got[1].zchi2, ref[1].zchi2) and torch.equal(got[1].zcoeff, ref[1].zcoeff)
+    assert float((got[0].zchi2 - ref[0].zchi2).abs().max()) <= 2e-5
+    chunked = zscan.scan_device(tg, dts, chunk=16)
+    for a, b in zip(chunked, got):
+        assert torch.equal(a.zchi2, b.zchi2) and torch.equal(a.zcoeff, b.zcoeff)
