@@ -50,6 +50,55 @@ __global__ void trapz_rebin_kernel(const double* __restrict__ x, int64_t nx,
   for (int b = 0; b < nb; ++b) o[b] = res[b];
 }
 
+template <int NB, bool DZ>
+__device__ __noinline__ bool rebin_bin_general(const double* __restrict__ x, int64_t nx,
+                                               const double* __restrict__ y, double zp1,
+                                               double e_lo, double e_hi, double (&res)[NB],
+                                               double (&dres)[DZ ? NB : 1]) {
+  double v[kMaxRebinBasis], dv[DZ ? kMaxRebinBasis : 1];
+  if (!rebin_bin_strided<DZ>(x, nx, y, nx, NB, zp1, e_lo, e_hi, v, dv)) return false;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) res[b] = v[b];
+  if (DZ)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) dres[b] = dv[b];
+  return true;
+}
+
+// The same for up to ten bases in registers (rebin_bin_reg); a warp's rows
+// leave through shared memory as one contiguous run.
+template <int NB>
+__global__ void __launch_bounds__(128) trapz_rebin_reg_kernel(
+    const double* __restrict__ x, int64_t nx, const double* __restrict__ y,
+    const double* __restrict__ edges, int64_t nbin, const double* __restrict__ z,
+    double* __restrict__ out, int* status) {
+  __shared__ double stage[128 * NB];
+  const int64_t ibin = blockIdx.x * (int64_t)128 + threadIdx.x;
+  const int64_t iz = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double res[NB], none[1];
+  if (ibin < nbin) {
+    const double zp1 = dadd(1.0, z[iz]);
+    const double lo = edges[ibin], hi = edges[ibin + 1];
+    bool exact = true;
+    bool in = rebin_bin_reg<NB>(x, nx, y, nx, zp1, lo, hi, first_above(x, nx, zp1, lo), res, exact,
+                                none);
+    if (in && !exact) in = rebin_bin_general<NB, false>(x, nx, y, zp1, lo, hi, res, none);
+    if (!in) {
+      set_status(status, RR_ERANGE);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) res[b] = nan("");
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) stage[threadIdx.x * NB + b] = res[b];
+  }
+  __syncwarp();
+  const int64_t first = blockIdx.x * (int64_t)128 + warp * 32;
+  const int n = (int)(nbin - first < 32 ? (nbin > first ? nbin - first : 0) : 32) * NB;
+  double* o = out + (iz * nbin + first) * NB;
+  for (int q = lane; q < n; q += 32) o[q] = stage[warp * 32 * NB + q];
+}
+
 // Fused builder for one grid: rebin + IGM into the padded basis layout.
 // Threads cover the padded pixel range [pix_offset - 5, pix_offset +
 // npix_pad + 5); pixels outside [pix_offset, pix_offset + npix) and basis
@@ -92,21 +141,6 @@ __global__ void build_basis_any_kernel(const double* __restrict__ x, int64_t nx,
 
 static __device__ __noinline__ double transmission_plain(int model, double z, double lobs) {
   return transmission(model, z, lobs);
-}
-
-template <int NB, bool DZ>
-__device__ __noinline__ bool rebin_bin_general(const double* __restrict__ x, int64_t nx,
-                                               const double* __restrict__ y, double zp1,
-                                               double e_lo, double e_hi, double (&res)[NB],
-                                               double (&dres)[DZ ? NB : 1]) {
-  double v[kMaxRebinBasis], dv[DZ ? kMaxRebinBasis : 1];
-  if (!rebin_bin_strided<DZ>(x, nx, y, nx, NB, zp1, e_lo, e_hi, v, dv)) return false;
-#pragma unroll
-  for (int b = 0; b < NB; ++b) res[b] = v[b];
-  if (DZ)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) dres[b] = dv[b];
-  return true;
 }
 
 // d/dz of the Inoue14 factor t (the other models' is 0 between their steps)
@@ -324,8 +358,19 @@ extern "C" int rr_trapz_rebin(const double* x, int64_t nx, const double* y, int6
   if (nz > 65535) return RR_ENOTSUP;
   dim3 block(128);
   dim3 grid((unsigned)((nbin + block.x - 1) / block.x), (unsigned)nz);
-  trapz_rebin_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
-      x, nx, y, (int)nbasis, edges, nbin, z, nz, out, nbin * nbasis, nbasis, status);
+  cudaStream_t st = (cudaStream_t)stream;
+#define RR_REBIN_CASE(N)                                                                          \
+  case N:                                                                                         \
+    trapz_rebin_reg_kernel<N><<<grid, block, 0, st>>>(x, nx, y, edges, nbin, z, out, status);     \
+    break;
+  switch (nbasis) {
+    RR_REBIN_CASE(1) RR_REBIN_CASE(2) RR_REBIN_CASE(3) RR_REBIN_CASE(4) RR_REBIN_CASE(5)
+    RR_REBIN_CASE(6) RR_REBIN_CASE(7) RR_REBIN_CASE(8) RR_REBIN_CASE(9) RR_REBIN_CASE(10)
+    default:
+      trapz_rebin_kernel<<<grid, block, 0, st>>>(x, nx, y, (int)nbasis, edges, nbin, z, nz, out,
+                                                 nbin * nbasis, nbasis, status);
+  }
+#undef RR_REBIN_CASE
   RR_CHECK_LAUNCH();
   return RR_OK;
 }

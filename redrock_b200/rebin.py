@@ -105,16 +105,19 @@ def rebin_template(template, myz, dwave=None, dedges=None, use_gpu=False, xmin=N
     if xmax is None:
         xmax = template.maxwave * (1 + zh.min())
     result = {}
+    # one upload of the template for all grids
+    if dwave or dedges:
+        twave, tflux = to_device(template.wave), to_device(template.flux)
     if dwave is not None:
         for hs, wave in dwave.items():
-            result[hs] = trapz_rebin(template.wave, template.flux, xnew=wave, myz=myz,
+            result[hs] = trapz_rebin(twave, tflux, xnew=wave, myz=myz,
                                      use_gpu=use_gpu, xmin=xmin, xmax=xmax)
     elif dedges is not None:
         for hs, edges in dedges.items():
             minedge = maxedge = None
             if type(edges) is tuple:
                 edges, minedge, maxedge = edges
-            result[hs] = trapz_rebin(template.wave, template.flux, edges=edges, myz=myz,
+            result[hs] = trapz_rebin(twave, tflux, edges=edges, myz=myz,
                                      use_gpu=use_gpu, xmin=xmin, xmax=xmax, edge_min=minedge,
                                      edge_max=maxedge)
     return result

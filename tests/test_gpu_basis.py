@@ -95,3 +95,25 @@ def test_build_igm_equals_rebin_times_transmission(model, order):
     t = transmission_Lyman(z, grid, model=model)
     want = O.trapz_rebin(wave, flux, xnew=grid, myz=z) * t[:, :, None]
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("nb,npix,nz", [(1, 33, 1), (3, 128, 2), (4, 129, 5), (8, 31, 3), (10, 300, 4),
+                                        (11, 65, 2)])
+def test_trapz_rebin_equals_oracle(nb, npix, nz):
+    """The drop-in rebin in registers (up to ten bases) and the general kernel
+    (eleven), and rebin_template's grids from one upload."""
+    from types import SimpleNamespace
+
+    from redrock_b200 import rebin
+    wave, flux = _template(nb, True, 200 + nb)
+    z = np.random.default_rng(nz).uniform(0.05, 2.0, nz)
+    grid = 3300.0 + np.cumsum(np.random.default_rng(1).choice([0.3, 1.1, 5.0, 9.0], size=npix))
+    want = O.trapz_rebin(wave, flux, xnew=grid, myz=z)
+    np.testing.assert_array_equal(rebin.trapz_rebin(wave, flux, xnew=grid, myz=z), want)
+    t = SimpleNamespace(wave=wave, flux=flux, minwave=wave[0], maxwave=wave[-1])
+    got = rebin.rebin_template(t, z, dwave={"a": grid, "b": grid[:20]})
+    np.testing.assert_array_equal(got["a"], want)
+    np.testing.assert_array_equal(got["b"], O.trapz_rebin(wave, flux, xnew=grid[:20], myz=z))
+    if nb == 1:
+        np.testing.assert_array_equal(rebin.trapz_rebin(wave * 1.3, flux[0], xnew=grid),
+                                      O.trapz_rebin(wave * 1.3, flux[0], xnew=grid))
