@@ -160,7 +160,7 @@ static __device__ __noinline__ double transmission_slope(double t, double z, dou
 // Per (z, pixel, basis) about 35 FP64 operations at two samples to a bin (135
 // with three full divisions).  Bound by its sample loads: L1 77 % busy, the
 // FP64 pipe 46 %.  GALAXY, 3311 x 7958 x 10: 3.60 -> 1.86 ms; QSO with
-// Inoue14, 3794 x 7958 x 4: 2.14 -> 1.33 ms (build_basis_any_kernel, one
+// Inoue14, 3794 x 7958 x 4: 2.14 -> 1.24 ms (build_basis_any_kernel, one
 // thread per (z, pixel), before).
 constexpr int kBuildThreads = 128;
 
@@ -181,9 +181,17 @@ struct BuildParams {
   int* status;    // RR_ERANGE there, or NULL
 };
 
+// Blocks per SM: small bases with Inoue14 are bound by the latency of its
+// chains (QSO 1.53 ms at three, 1.34 at four, 1.24 at six), without it, and
+// for large ones, fewer registers cost more (five STAR bases 8 % at six;
+// GALAXY 1.92 / 1.85 / 2.83 ms).
+constexpr int build_blocks(int nb, bool inoue, bool dz) {
+  return dz ? 3 : (nb <= 5 && inoue ? 6 : 4);
+}
+
 // INOUE: the Inoue14 factor; else the other models, or none.  DZ: dT/dz too.
 template <int NB, bool INOUE, bool DZ>
-__global__ void __launch_bounds__(kBuildThreads, (DZ ? 3 : 4)) build_basis_kernel(
+__global__ void __launch_bounds__(kBuildThreads, build_blocks(NB, INOUE, DZ)) build_basis_kernel(
     const __grid_constant__ BuildParams p) {
   constexpr int S = (NB + 1) & ~1;
   constexpr int kZ = build_z(INOUE);
