@@ -35,22 +35,33 @@ BLOCK_GROUPS = (0, 4)
 _cache = {}
 
 
-def _key(pack, bases):
+def _blocks(pack, tail):
+    """Target blocks of the pack that the fused launch scans."""
+    return pack.nblock if not tail else -(-(pack.ntarget - tail) // 32)
+
+
+def _key(pack, bases, tail):
     small = tuple(sorted((b.nbasis, b.nz) for b in bases if b.nbasis in CANDIDATES))
     nb = 1
-    while nb < pack.nblock:
+    while nb < _blocks(pack, tail):
         nb *= 2
     return (pack.layout.signature, small, nb)
 
 
-def choice(pack, bases):
-    return _cache.get(_key(pack, bases))
+def choice(pack, bases, tail=0):
+    return _cache.get(_key(pack, bases, tail))
 
 
-def tune(pack, bases, repeats=1):
-    """Time the candidates and cache the fastest ZT per small nbasis."""
-    from .engine import run_fused
-    key = _key(pack, bases)
+def tune(pack, bases, repeats=1, tail=0):
+    """Time the candidates and cache the fastest ZT per small nbasis.  tail:
+    the pack's last targets that the few-target kernel takes (not timed: with
+    one fused block of a 48-target batch QSO is fastest at two redshifts per
+    thread, with two at one)."""
+    from .engine import run_fused as _run
+
+    def run_fused(*a, **kw):
+        return _run(*a, tail=tail, scan_tail=False, **kw)
+    key = _key(pack, bases, tail)
     if key in _cache:
         return _cache[key]
     best = {}
@@ -60,27 +71,27 @@ def tune(pack, bases, repeats=1):
             continue
         times = {}
         for zt in cands:
-            run_fused(pack, sub, tiles={nb: zt}, tail=0)   # untimed (first launch of a variant)
+            run_fused(pack, sub, tiles={nb: zt})   # untimed (first launch of a variant)
             ev = []
             for _ in range(repeats):
-                run_fused(pack, sub, tiles={nb: zt}, kernel_events=ev, tail=0)
+                run_fused(pack, sub, tiles={nb: zt}, kernel_events=ev)
             torch.cuda.synchronize()
             times[zt] = sum(a.elapsed_time(b) for a, b in ev) / len(ev)
         best[nb] = min(times, key=times.get)
         best[f"ms_{nb}"] = {zt: round(t, 3) for zt, t in times.items()}
     # tile order, timed on the templates without a ZT choice (GALAXY's
     # nbasis 10: the bulk of the scan), else on all of them
-    groups = [g for g in BLOCK_GROUPS if g == 0 or g < pack.nblock]
+    groups = [g for g in BLOCK_GROUPS if g == 0 or g < _blocks(pack, tail)]
     if len(groups) > 1:
         sub = [b for b in bases if b.nbasis not in CANDIDATES] or list(bases)
         zt = {nb: best[nb] for nb in CANDIDATES if nb in best}
         times = {}
         for g in groups:
             tiles = dict(zt, block_group=g)
-            run_fused(pack, sub, tiles=tiles, tail=0)
+            run_fused(pack, sub, tiles=tiles)
             ev = []
             for _ in range(repeats):
-                run_fused(pack, sub, tiles=tiles, kernel_events=ev, tail=0)
+                run_fused(pack, sub, tiles=tiles, kernel_events=ev)
             torch.cuda.synchronize()
             times[g] = sum(a.elapsed_time(b) for a, b in ev) / len(ev)
         best["block_group"] = min(times, key=times.get)

@@ -593,13 +593,14 @@ class FewRows:
 
 
 def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=None,
-              tiles=None, external_events=False, tail=None, ntarget=None):
+              tiles=None, external_events=False, tail=None, ntarget=None, scan_tail=True):
     """One persistent launch over every (target, template, z).  ygemm:
     None (DEFAULT_Y, or "fp64" for the templates y_in_scan says), "fp64", "int8x6",
     "int8x7", "bf16x3" or "tf32x3"; other than
     "fp64", y is computed on the tensor cores first (YGemm).  ntarget: the size
     of the whole batch when the pack is a chunk of it (y_in_scan's choice must
-    not depend on the chunks).  kernel_events:
+    not depend on the chunks).  scan_tail=False leaves the tail's results
+    unwritten (the tuner's launches).  kernel_events:
     a list that gets a (start, end) CUDA event pair around the scan launches
     alone (timing).  tiles: redshifts per thread {nbasis: ZT} for the small
     bases (nbasis 4: 1-3, nbasis 5: 1-2; rr_scan_options) and optionally
@@ -620,7 +621,7 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
                         and b.stride == round_up(b.nbasis, 2) for b in bases)
         tail = few_tail(pack.ntarget) if ygemm is None and plain_pca else 0
     nfull = pack.ntarget - tail
-    few = FewRows(pack, nfull, tail, stream=stream) if tail else None
+    few = FewRows(pack, nfull, tail, stream=stream) if tail and scan_tail else None
     fused = nfull > 0 or not tail
     rows = None
     if fused:

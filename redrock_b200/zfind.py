@@ -381,9 +381,10 @@ class _PackShape:
     """What the tile autotuner keys a choice on (grid layout, number of
     target blocks), without packing the targets."""
 
-    def __init__(self, layout, nblock):
+    def __init__(self, layout, nblock, ntarget):
         self.layout = layout
         self.nblock = nblock
+        self.ntarget = ntarget
 
 
 class DeviceFitzPlan:
@@ -419,11 +420,12 @@ class DeviceFitzPlan:
                      for t in self.templates]
         self.dbatch = TargetBatch(local, layout).to_device()
         self.rowpack = RowPack(self.dbatch)
-        key = _PackShape(layout, self.dbatch.batch.nblock)
-        best = autotune.choice(key, self.bases)
-        if best is None and few_tail(len(local)) < len(local):
+        tail = few_tail(len(local))
+        key = _PackShape(layout, self.dbatch.batch.nblock, len(local))
+        best = autotune.choice(key, self.bases, tail)
+        if best is None and tail < len(local):
             pack0 = TargetPack(self.dbatch, status=self.status)
-            best = autotune.tune(pack0, self.bases)
+            best = autotune.tune(pack0, self.bases, tail=tail)
             del pack0
         self.tiles = autotune.tiles_of(best)
         dev = torch.cuda.current_device()

@@ -375,8 +375,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
             tail = max(0, i1 - max(i0, few0))
             if AUTOTUNE and tail < len(sub):
                 from . import autotune
-                tiles = autotune.tiles_of(autotune.choice(pack, bases)
-                                          or autotune.tune(pack, bases))
+                tiles = autotune.tiles_of(autotune.choice(pack, bases, tail)
+                                          or autotune.tune(pack, bases, tail=tail))
             res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=tail,
                                ntarget=len(targets))
         keep.append((pack, res))
