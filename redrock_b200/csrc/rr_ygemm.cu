@@ -601,16 +601,23 @@ __global__ void __launch_bounds__(kThreads, 1) ygemm_kernel(const __grid_constan
         break;
       }
       tc_fence_after();
-      const uint32_t a0 = smem_u32(sm + s * Gm::kStageBytes);
-      const uint32_t b0 = a0 + Gm::kABlock;
-#pragma unroll 1
+      // the descriptors of a stage's planes differ by constants in their
+      // address field (16-byte units; all of shared memory fits its 14 bits),
+      // so with the loops unrolled a product costs its issuing thread a few
+      // instructions; formed one by one they took longer (127 cycles per
+      // product) than the tensor core (42 at N = 80).  GALAXY at 448 targets
+      // 4.09 -> 2.32 ms, QSO 2.06 -> 1.18; what bounds a product now, about 70
+      // cycles, is its 6.5 KB of operands out of shared memory and their
+      // refill.
+      const uint64_t da0 = smem_desc(smem_u32(sm + s * Gm::kStageBytes), kSbo);
+      const uint64_t db0 = smem_desc(smem_u32(sm + s * Gm::kStageBytes) + Gm::kABlock, kSbo);
+#pragma unroll
       for (int d = 0; d < S::kDigits; ++d)
-#pragma unroll 1
-        for (int i = 0; i <= d; ++i) {
-          const uint64_t da = smem_desc(a0 + i * kASlice, kSbo);
-          const uint64_t db = smem_desc(b0 + (d - i) * Gm::kBSlice, kSbo);
-          mma<kI8>(tmem + d * kN, da, db, idesc, (c > 0 || i > 0) ? 1u : 0u);
-        }
+#pragma unroll
+        for (int i = 0; i <= d; ++i)
+          mma<kI8>(tmem + d * kN, da0 + (uint64_t)(i * kASlice / 16),
+                   db0 + (uint64_t)((d - i) * Gm::kBSlice / 16), idesc,
+                   (c > 0 || i > 0) ? 1u : 0u);
       mma_commit(&empty[s]);
     }
     mma_commit(&acc_done);

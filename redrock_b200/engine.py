@@ -520,16 +520,16 @@ def y_in_scan(basis, ntarget):
     """Whether y of a batch of ntarget targets against this basis is cheaper
     summed inside the scan (FP64) than as a tensor-core GEMM of its own.
     The GEMM takes rounds of one 128-target x 80-column tile per SM, each as
-    long as the pixels are (0.33 ms for 8064), however few tiles there are:
-    five STAR templates of 100 redshifts cost it 1.7 ms at any batch up to
+    long as the pixels are (0.19 ms for 8064), however few tiles there are:
+    five STAR templates of 100 redshifts cost it 0.95 ms at any batch up to
     1000 targets.  The scan sums y at 13 TFMA/s; ten bases leave it no
-    registers for y and pay about twice that (32 targets: GALAXY 11.4 ms with
-    the GEMM and 12.0 without, QSO 5.7 and 5.3, STAR 3.5 and 1.9; the QSO lines
-    cross between 64 and 96 targets, 10.2 / 10.0 and 13.0 / 13.2 ms)."""
+    registers for y and pay about twice that.  With the GEMM and without, ms:
+    32 targets GALAXY 10.96 / 11.97, QSO 5.43 / 5.35, STAR 2.81 / 1.90; 64
+    targets QSO 9.89 / 10.04; 128 targets STAR 4.32 / 3.46."""
     L = _lib.lib()
     kpad = int(L.rr_ygemm_kpad(basis.layout.pix_stride))
     tiles = -(-basis.nz // (80 // basis.nbasis)) * -(-ntarget // 128)
-    gemm = -(-tiles // 148) * (kpad / 32) * 1.32e-6
+    gemm = -(-tiles // 148) * (kpad / 32) * 0.76e-6
     lanes = round_up(max(ntarget, 1), _lib.LANES)
     scan = lanes * basis.nz * basis.layout.pix_stride * basis.nbasis / 13.3e12
     return scan * (2.3 if basis.nbasis > 5 else 1.0) < gemm
