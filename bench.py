@@ -221,7 +221,9 @@ def run_ours(args, rank, world, local_rank):
     evals, flops, y_flops = evals_and_flops(rtg, tms)
     layout = GridLayout.from_dwave(synth.camera_grids())
     if args.ygemm is None:
-        # the engine's own choice for this layout (what the public API runs)
+        # the engine's y variant for this layout, for every template and all
+        # targets; the public API (e2e) also sums y in the scan for small
+        # templates and gives a batch's last targets to the few-target scan
         from redrock_b200.engine import resolve_y
         args.ygemm = resolve_y(None, layout)
     srcs = [TemplateSource.from_template(tm) for tm in tms]
@@ -284,7 +286,7 @@ def run_ours(args, rank, world, local_rank):
     # template
     groups = {0 if tm.nbasis == 10 else 1 if tm.nbasis == 4 else 2 if tm.nbasis == 5 else 3
               for tm in tms}
-    launches_per_step = sum(len(layout.keys) for _ in srcs) + 2 + len(groups)
+    launches_per_step = len(srcs) + 2 + len(groups)
     if args.ygemm in ("int8x7", "int8x6"):
         # rr_pack_g, rr_slice_g_i8; per template rr_basis_col_exp,
         # rr_slice_basis_i8, rr_ygemm_i8

@@ -78,10 +78,10 @@ enum rr_solve_method { /* zscan.py:1107-1203 solve_matrices */
   RR_SOLVE_UNSUPPORTED = 1, /* every z gets HUGE_CHI2 and zero coefficients,
                               as redrock does for NotImplementedError */
   RR_SOLVE_NNLS = 2,       /* NMF / NNLS: min ||M c - y||, c >= 0 (scipy nnls
-                              on (M, y), zscan.py:1153-1169); plain path only */
+                              on (M, y), zscan.py:1153-1169); not in the fused scan */
   RR_SOLVE_BVLS = 3        /* min ||M c - y||, lo <= c <= hi (scipy lsq_linear
-                              method='bvls', zscan.py:1170-1199); plain path
-                              only (rr_zchi2_batch_plain_ex) */
+                              method='bvls', zscan.py:1170-1199); not in the
+                              fused scan */
 };
 
 #define RR_HUGE_CHI2 9999999.0   /* zscan.py:18 */

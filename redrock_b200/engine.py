@@ -644,14 +644,15 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
             for b, r, ins in zip(sub, out, inside[i0:]):
                 # kept with the result so it outlives the launch
                 r.y_ext = yg.y(b, stream=stream) if yg is not None and not ins else None
+        if kernel_events is not None:
+            # external events become event-record nodes when the launches
+            # are captured in a CUDA graph, so each replay times them
+            e0 = torch.cuda.Event(enable_timing=True, external=external_events)
+            e1 = torch.cuda.Event(enable_timing=True, external=external_events)
+            _record(e0, stream)
+        if fused:
             tms = _scan_templates(sub, out)
             arr = (_lib.ScanTemplate * len(tms))(*tms)
-            if kernel_events is not None:
-                # external events become event-record nodes when the launches
-                # are captured in a CUDA graph, so each replay times them
-                e0 = torch.cuda.Event(enable_timing=True, external=external_events)
-                e1 = torch.cuda.Event(enable_timing=True, external=external_events)
-                _record(e0, stream)
             if tiles:
                 opt = _lib.ScanOptions(int(tiles.get(4, 0)), int(tiles.get(5, 0)),
                                        int(tiles.get("block_group", 0)))
@@ -661,12 +662,11 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
                 rc = L.rr_zscan_fused(ctypes.byref(tgs), arr, len(tms), ptr(counter), st.ptr,
                                       stream_handle(stream))
             _lib.check(rc, "rr_zscan_fused")
-            if kernel_events is not None:
-                _record(e1, stream)
-                kernel_events.append((e0, e1))
         if few is not None:
-            few.scan(sub, out, counter, st, after_fused=fused and kernel_events is None,
-                     stream=stream)
+            few.scan(sub, out, counter, st, after_fused=fused, stream=stream)
+        if kernel_events is not None:
+            _record(e1, stream)
+            kernel_events.append((e0, e1))
     for r in results[:1]:
         r.few = (few, rows)   # outlive the launches
     run_fused.last_counter = counter
@@ -735,10 +735,18 @@ PAIR_WS_BYTES = 1 << 30
 
 
 def _pair_ws(nbytes, segs, nbasis, n, dev):
-    """Workspace of n pairs, at most PAIR_WS_BYTES (but two pairs)."""
+    """Workspace of n pairs, at most PAIR_WS_BYTES (but two pairs); less, and
+    so more rounds, when the device has not that much left."""
     need = int(nbytes(segs, len(segs), nbasis, n + n % 2))
     two = int(nbytes(segs, len(segs), nbasis, 2))
-    return torch.empty(min(need, max(two, PAIR_WS_BYTES)), dtype=torch.uint8, device=dev)
+    size = min(need, max(two, PAIR_WS_BYTES))
+    while True:
+        try:
+            return torch.empty(size, dtype=torch.uint8, device=dev)
+        except torch.cuda.OutOfMemoryError:
+            if size <= two:
+                raise
+            size = max(two, size // 4)
 
 
 def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream):

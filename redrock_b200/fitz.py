@@ -7,8 +7,8 @@ between its neighbours, fit a parabola to the three points around the best
 one, fit the template once more at the parabola minimum, set ZWARN bits, and
 return the results sorted by chi2.
 
-All chi2 evaluations run in the pair-scan kernel (``rr_zscan_pairs``): one
-launch per template evaluates the fine grids of every target's candidate
+All chi2 evaluations run in the pair scan (``rr_zscan_pairs_ws``): one
+call per template evaluates the fine grids of every target's candidate
 minima (each target at its own redshifts), and one more launch does the
 single-z fits at the parabola minima.  Templates with a bounded solve (NMF /
 NNLS / BVLS) use the same launches with the kernel's bounded solvers and

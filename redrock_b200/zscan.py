@@ -187,10 +187,11 @@ def _bounded_scan(targets, basis, layout):
     take about 1 MB each).  Targets it cannot take -- a negative or NaN
     weight, whose square root the packed rows hold, or more spectra on a
     grid than a pack has segments for -- go through the plain per-target
-    chain."""
+    chain, as does a basis with another row stride."""
     from .device import StatusWord
     plain = [i for i, t in enumerate(targets)
-             if not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
+             if basis.stride != basis.nbasis + basis.nbasis % 2
+             or not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
     few = [i for i in range(len(targets)) if i not in set(plain)]
     res = ScanResult(len(targets), basis, torch.device("cuda", torch.cuda.current_device()))
     st = StatusWord()
@@ -338,7 +339,9 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     st = StatusWord()
     bounds = _chunk_bounds(len(targets), chunk)
     # the last targets that fill no block, whatever chunk they fall into
-    few0 = len(targets) - few_tail(len(targets))
+    few0 = len(targets)
+    if all(b.stride == b.nbasis + b.nbasis % 2 for b in bases):
+        few0 -= few_tail(len(targets))
     main = torch.cuda.current_stream()
     # consecutive chunks alternate between two compute streams, so that a
     # chunk's packing, y GEMMs and first scan launch need not wait for the
