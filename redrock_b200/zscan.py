@@ -349,11 +349,13 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     # chunk's last tile wave leaves idle (each chunk has its own outputs,
     # tile counters and scratch, allocated on its own stream)
     lanes = [main] if len(bounds) == 1 else [main, _lane_stream()]
-    if len(lanes) > 1 and few0 > 0:
-        # what the chunks share is made on main first: the bases and their
-        # INT8 digit planes for the y GEMM (cached on each basis)
+    if len(lanes) > 1:
+        # what the chunks share is made on main first: the bases, the status
+        # word and, where a chunk has targets for the fused scan, the INT8
+        # digit planes for the y GEMM (cached on each basis).  The lane
+        # waits for main in every case.
         yv = _lib.YGEMM_VARIANTS[resolve_y(None, layout)]
-        if yv in _lib.I8_VARIANTS:
+        if few0 > 0 and yv in _lib.I8_VARIANTS:
             kpad = int(_lib.lib().rr_ygemm_kpad(layout.pix_stride))
             for b in bases:
                 if not y_in_scan(b, len(targets)):
