@@ -535,6 +535,20 @@ def y_in_scan(basis, ntarget):
     return scan * (2.3 if basis.nbasis > 5 else 1.0) < gemm
 
 
+def _use_on(stream, *tensors):
+    """Buffers that a call made on the current stream for its launches on
+    ``stream``: where that is another stream, its work from here on waits
+    for what the current one has queued (their filling, and whatever used
+    their memory before), and their memory is not given out again before it
+    is done."""
+    if stream is None or stream == torch.cuda.current_stream():
+        return
+    stream.wait_stream(torch.cuda.current_stream())
+    for t in tensors:
+        if t is not None:
+            t.record_stream(stream)
+
+
 def _record(ev, stream):
     if isinstance(stream, torch.cuda.Stream):
         ev.record(stream)
@@ -576,6 +590,7 @@ class FewRows:
         if n < 0:
             raise ValueError("target segments do not fit the few-target scan")
         self.lrows = torch.empty(count * n, dtype=torch.float64, device=pack.rw.device)
+        _use_on(stream, self.lrows)
         rc = L.rr_pack_few(ctypes.byref(self.tgs), first, count, ptr(self.lrows),
                            stream_handle(stream))
         _lib.check(rc, "rr_pack_few")
@@ -630,6 +645,7 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
             # the last fused block also holds targets of the tail: not its rows
             rows = pack.rows.clone()
             rows[nfull:] = -1
+        _use_on(stream, counter, rows)
         tgs = pack.scan_targets_struct(nblock, rows)
         inside = [False] * len(bases)
         if ygemm is None:
@@ -754,6 +770,7 @@ def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, stat
     L = _lib.lib()
     nseg = len(rowpack.segments)
     ws = _pair_ws(L.rr_zscan_pairs_ws_bytes, segs, tm.nbasis, n, chi2.device)
+    _use_on(stream, ws, pair_target, pair_z)
     rc = L.rr_zscan_pairs_ws(ctypes.byref(tm), segs, nseg, ptr(rowpack.rows), ptr(rowpack.fwf),
                              ptr(rowpack.wsum), rowpack.npix_row, ptr(pair_target), ptr(pair_z), n,
                              ptr(chi2), ptr(coeff), ptr(pen), ptr(ws), ws.numel(), status.ptr,
@@ -867,6 +884,7 @@ def run_pairs_grad(rowpack, src, pair_target, pair_z, want_dflux=False, stream=N
     segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
     st = status or StatusWord(dev)
     ws = _pair_ws(L.rr_zscan_pairs_grad_ws_bytes, segs, nb, n, dev)
+    _use_on(stream, ws, dt, dz)
     rc = L.rr_zscan_pairs_grad_ws(ctypes.byref(tm), segs, len(rowpack.segments),
                                   ptr(rowpack.rows), ptr(rowpack.sw), ptr(rowpack.fwf),
                                   ptr(rowpack.wsum), rowpack.npix_row, ptr(dt), ptr(dz), n,
