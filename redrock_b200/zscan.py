@@ -180,38 +180,42 @@ class HostResult:
 _FUSED_METHODS = (_lib.RR_SOLVE_PCA, _lib.RR_SOLVE_UNSUPPORTED)
 
 
-def _bounded_scan(targets, basis, layout):
-    """One template with a bounded solve (calc_zchi2's loop, zscan.py:853-887)
+def _bounded_scan(targets, bases, layout):
+    """Templates with a bounded solve (calc_zchi2's loop, zscan.py:853-887)
     for every target, results on the device like the fused scan's: the
     few-target kernel, BOUNDED_CHUNK targets at a time (their packed rows
-    take about 1 MB each).  Targets it cannot take -- a negative or NaN
-    weight, whose square root the packed rows hold, or more spectra on a
-    grid than a pack has segments for -- go through the plain per-target
-    chain, as does a basis with another row stride."""
+    take about 1 MB each), packed anew in every call, so that a target whose
+    arrays were changed in place is read as it is now.  Targets it cannot
+    take -- a negative or NaN weight, whose square root the packed rows hold,
+    or more spectra on a grid than a pack has segments for -- go through the
+    plain per-target chain, as does a basis with another row stride."""
     from .device import StatusWord
+    dev = torch.device("cuda", torch.cuda.current_device())
+    res = [ScanResult(len(targets), b, dev) for b in bases]
+    even = [k for k, b in enumerate(bases) if b.stride == b.nbasis + b.nbasis % 2]
     plain = [i for i, t in enumerate(targets)
-             if basis.stride != basis.nbasis + basis.nbasis % 2
-             or not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
-    few = [i for i in range(len(targets)) if i not in set(plain)]
-    res = ScanResult(len(targets), basis, torch.device("cuda", torch.cuda.current_device()))
+             if not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
+    few = [i for i in range(len(targets)) if i not in set(plain)] if even else []
     st = StatusWord()
-    counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=res.zchi2.device)
+    counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=dev)
     for i0 in range(0, len(few), BOUNDED_CHUNK):
         ix = few[i0:i0 + BOUNDED_CHUNK]
-        part = [targets[i] for i in ix]
         try:
-            pack = _pack(part, layout) if len(ix) == len(targets) else \
-                TargetPack.from_targets(part, layout)
+            pack = TargetPack.from_targets([targets[i] for i in ix], layout)
         except NotImplementedError:
             plain += ix
             continue
         if len(ix) < len(targets):
             pack.rows[:len(ix)] = torch.as_tensor(ix, dtype=torch.int32).to(pack.rows.device)
-        FewRows(pack, 0, len(ix)).scan([basis], [res], counter, st)
+        rows = FewRows(pack, 0, len(ix))
+        for k0 in range(0, len(even), _lib.MAX_TEMPLATES):
+            sub = even[k0:k0 + _lib.MAX_TEMPLATES]
+            rows.scan([bases[k] for k in sub], [res[k] for k in sub], counter, st)
         pack.check()
     st.check("rr_zscan_few")
-    for i in plain:
-        _plain_target(targets[i], basis, layout, res, i)
+    for k, b in enumerate(bases):
+        for i in plain if k in even else range(len(targets)):
+            _plain_target(targets[i], b, layout, res[k], i)
     return res
 
 
@@ -324,8 +328,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
             part = scan_device(targets, [dtemplates[i] for i in fused_ix], chunk=chunk, host=host)
             for i, r in zip(fused_ix, part):
                 out[i] = r
-        for i in plain_ix:
-            r = _bounded_scan(targets, all_bases[i], layout)
+        for i, r in zip(plain_ix, _bounded_scan(targets, [all_bases[i] for i in plain_ix],
+                                                layout)):
             if host:
                 h = HostResult(len(targets), all_bases[i])
                 for dst, src in zip(h.t, (r.zchi2, r.zcoeff, r.penalty)):
