@@ -186,15 +186,15 @@ def _bounded_scan(targets, bases, layout):
     few-target kernel, BOUNDED_CHUNK targets at a time (their packed rows
     take about 1 MB each), packed anew in every call, so that a target whose
     arrays were changed in place is read as it is now.  Targets it cannot
-    take -- a negative or NaN weight, whose square root the packed rows hold,
-    or more spectra on a grid than a pack has segments for -- go through the
+    take -- a negative or non-finite weight, whose square root the packed
+    rows hold (times the zeros outside the band: NaN for an infinite one), or
+    more spectra on a grid than a pack has segments for -- go through the
     plain per-target chain, as does a basis with another row stride."""
     from .device import StatusWord
     dev = torch.device("cuda", torch.cuda.current_device())
     res = [ScanResult(len(targets), b, dev) for b in bases]
     even = [k for k, b in enumerate(bases) if b.stride == b.nbasis + b.nbasis % 2]
-    plain = [i for i, t in enumerate(targets)
-             if not all(np.all(np.asarray(s.ivar) >= 0) for s in t.spectra)]
+    plain = [i for i, t in enumerate(targets) if not all(_weights_ok(s.ivar) for s in t.spectra)]
     few = [i for i in range(len(targets)) if i not in set(plain)] if even else []
     st = StatusWord()
     counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=dev)
@@ -217,6 +217,12 @@ def _bounded_scan(targets, bases, layout):
         for i in plain if k in even else range(len(targets)):
             _plain_target(targets[i], b, layout, res[k], i)
     return res
+
+
+def _weights_ok(ivar):
+    """Whether the packed rows can hold the square root of these weights."""
+    w = np.asarray(ivar)
+    return bool(np.all((w >= 0) & (w < np.inf)))
 
 
 def _plain_target(t, basis, layout, res, i):

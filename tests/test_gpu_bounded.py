@@ -43,3 +43,21 @@ def test_flux_changed_in_place():
         ref = zscan.calc_zchi2([t.id for t in fresh], fresh, dt)
         for x, y in zip((g.zchi2, g.zcoeff, g.penalty), ref):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("weight", [np.inf, np.nan, -0.5])
+def test_weights_without_a_square_root(weight):
+    """A target with a weight that the packed rows cannot hold keeps the
+    plain chain's results; the others of its batch keep theirs."""
+    from redrock_b200 import synth, templates as TM, zscan
+    from redrock_b200.engine import ScanResult
+    dt = TM.DistTemplate(_nmf(5), synth.camera_grids())
+    tg = _targets(3)
+    clean = zscan.calc_zchi2([t.id for t in tg], tg, dt)
+    tg[1].spectra[0].ivar[100] = weight
+    got = zscan.calc_zchi2([t.id for t in tg], tg, dt)
+    ref = ScanResult(3, dt.basis, dt.basis.basis.device)
+    zscan._plain_target(tg[1], dt.basis, dt.layout, ref, 1)
+    for x, y, z in zip(got, clean, (ref.zchi2, ref.zcoeff, ref.penalty)):
+        np.testing.assert_array_equal(x[1], z.cpu().numpy()[1])
+        np.testing.assert_array_equal(x[[0, 2]], y[[0, 2]])
