@@ -194,8 +194,9 @@ def _bounded_scan(targets, bases, layout):
     dev = torch.device("cuda", torch.cuda.current_device())
     res = [ScanResult(len(targets), b, dev) for b in bases]
     even = [k for k, b in enumerate(bases) if b.stride == b.nbasis + b.nbasis % 2]
-    plain = [i for i, t in enumerate(targets) if not all(_weights_ok(s.ivar) for s in t.spectra)]
-    few = [i for i in range(len(targets)) if i not in set(plain)] if even else []
+    ok = [all(_weights_ok(s.ivar) for s in t.spectra) for t in targets]
+    plain = [i for i, o in enumerate(ok) if not o]
+    few = [i for i, o in enumerate(ok) if o] if even else []
     st = StatusWord()
     counter = torch.zeros(_lib.FUSED_COUNTERS, dtype=torch.int32, device=dev)
     for i0 in range(0, len(few), BOUNDED_CHUNK):
