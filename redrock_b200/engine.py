@@ -765,11 +765,22 @@ def _pair_ws(nbytes, segs, nbasis, n, dev):
             size = max(two, size // 4)
 
 
-def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream):
-    """rr_zscan_pairs_ws over device pairs, in rounds of PAIR_WS_BYTES."""
+def pair_workspace(rowpack, sources, n):
+    """One workspace for pair scans (run_pairs_device) of up to n pairs of
+    each of these templates, one after another on one stream."""
+    segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
+    return _pair_ws(_lib.lib().rr_zscan_pairs_ws_bytes, segs, max(s.nbasis for s in sources), n,
+                    rowpack.rows.device)
+
+
+def _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream,
+               ws=None):
+    """rr_zscan_pairs_ws over device pairs, in as many rounds as the
+    workspace takes (its own, of up to PAIR_WS_BYTES, when none is given)."""
     L = _lib.lib()
     nseg = len(rowpack.segments)
-    ws = _pair_ws(L.rr_zscan_pairs_ws_bytes, segs, tm.nbasis, n, chi2.device)
+    if ws is None:
+        ws = _pair_ws(L.rr_zscan_pairs_ws_bytes, segs, tm.nbasis, n, chi2.device)
     _use_on(stream, ws, pair_target, pair_z)
     rc = L.rr_zscan_pairs_ws(ctypes.byref(tm), segs, nseg, ptr(rowpack.rows), ptr(rowpack.fwf),
                              ptr(rowpack.wsum), rowpack.npix_row, ptr(pair_target), ptr(pair_z), n,
@@ -811,10 +822,12 @@ def run_pairs(rowpack, src, pair_target, pair_z, stream=None, status=None, bound
     return chi2, coeff, pen
 
 
-def run_pairs_device(rowpack, src, pair_target, pair_z, status, stream=None):
+def run_pairs_device(rowpack, src, pair_target, pair_z, status, stream=None, ws=None):
     """run_pairs for pairs already on the device (int32 target indices and
     float64 redshifts, both CUDA tensors); stays asynchronous (the caller's
-    status word reports kernel errors), so it can be captured in a graph."""
+    status word reports kernel errors), so it can be captured in a graph.
+    ws: a workspace to use (pair_workspace) instead of one of its own, which
+    under capture would stay in the graph's memory pool."""
     L = _lib.lib()
     dev = device()
     n = int(pair_z.numel())
@@ -828,7 +841,7 @@ def run_pairs_device(rowpack, src, pair_target, pair_z, status, stream=None):
     tm = _lib.PairTemplate(ptr(src.x), src.nx, ptr(src.y), nb, src.igm, src.method, 0,
                            ptr(prior), ptr(src.oii_dev))
     segs = (_lib.PairSegment * len(rowpack.segments))(*rowpack.segments)
-    _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream)
+    _pair_scan(rowpack, tm, segs, pair_target, pair_z, n, chi2, coeff, pen, status, stream, ws)
     return chi2, coeff, pen
 
 

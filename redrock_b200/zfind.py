@@ -406,7 +406,8 @@ class DeviceFitzPlan:
         import torch
         from . import autotune
         from .device import StatusWord, to_device
-        from .engine import TargetBatch, TargetPack, TemplateSource, few_tail, run_fused
+        from .engine import (TargetBatch, TargetPack, TemplateSource, few_tail, pair_workspace,
+                             run_fused)
         from .zscan import _bases_for
         self.local = local
         self.templates = list(templates)
@@ -420,6 +421,10 @@ class DeviceFitzPlan:
                      for t in self.templates]
         self.dbatch = TargetBatch(local, layout).to_device()
         self.rowpack = RowPack(self.dbatch)
+        # the templates' fine-grid scans follow one another on one stream,
+        # so they share a workspace, made outside the graphs' memory pools
+        # (in them it would be kept once per template: 7 GB for the seven)
+        self.pair_ws = pair_workspace(self.rowpack, self.srcs, len(local) * self.K * nfine)
         tail = few_tail(len(local))
         key = _PackShape(layout, self.dbatch.batch.nblock, len(local))
         best = autotune.choice(key, self.bases, tail)
@@ -472,7 +477,8 @@ class DeviceFitzPlan:
         b = self.bases[k]
         fc = FitzCandidates(r.zchi2, r.penalty if b.oii is not None else None, self.zdev[k],
                             self.K, self.nfine)
-        c2, _, pen = run_pairs_device(rowpack, self.srcs[k], fc.pair_t, fc.pair_z, self.status)
+        c2, _, pen = run_pairs_device(rowpack, self.srcs[k], fc.pair_t, fc.pair_z, self.status,
+                                      ws=self.pair_ws)
         return fc, c2, pen
 
     def launch(self):
