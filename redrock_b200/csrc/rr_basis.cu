@@ -149,14 +149,14 @@ static __device__ __noinline__ double transmission_slope(double t, double z, dou
 }
 
 // The builder for basis rows of NB values (rounded up to even), all grids in
-// one launch: a block takes 128 padded pixels and build_z redshifts, a thread
-// one pixel for all of them, with the bases in registers.  What a pixel and
-// what a redshift need of the IGM is then formed once (InoueWave, InoueZ)
+// one launch: a block takes 128 padded pixels and up to build_z redshifts, a
+// thread one pixel for all of them, with the bases in registers.  What a pixel
+// and what a redshift need of the IGM is then formed once (InoueWave, InoueZ)
 // instead of once per (z, pixel) -- 16 redshifts to a block with Inoue14, 4
-// without, where more would only leave the last wave of blocks emptier --,
-// the divisions share their reciprocals (rebin_bin_reg) and the
-// rows leave through shared memory as whole 16-byte columns of a warp's 32
-// consecutive rows.
+// without, where more would only leave the last wave of blocks emptier, and
+// fewer than 16 on short redshift grids (build_per_block) --, the divisions
+// share their reciprocals (rebin_bin_reg) and the rows leave through shared
+// memory as whole 16-byte columns of a warp's 32 consecutive rows.
 // Per (z, pixel, basis) about 35 FP64 operations at two samples to a bin (135
 // with three full divisions).  Bound by its sample loads: L1 77 % busy, the
 // FP64 pipe 46 %.  GALAXY, 3311 x 7958 x 10: 3.60 -> 1.86 ms; QSO with
@@ -174,6 +174,7 @@ struct BuildParams {
   int first[kBuildGrids + 1];  // first block of each grid
   int ngrid;
   int igm_model;
+  int kz;  // redshifts per block with Inoue14
   double* basis;
   double* dbasis;  // dT/dz in the same layout (DZ)
   int64_t pix_stride;
@@ -204,8 +205,9 @@ __global__ void __launch_bounds__(kBuildThreads, build_blocks(NB, INOUE, DZ)) bu
   const int64_t bx = blockIdx.x - p.first[ig];
   const int64_t span = gd.npix_pad + 2 * kHalfBand;
   const int64_t i = bx * kBuildThreads + threadIdx.x;
-  const int64_t z0 = blockIdx.y * (int64_t)kZ;
-  const int nz = (int)(p.nz - z0 < kZ ? p.nz - z0 : kZ);
+  const int per = INOUE ? p.kz : kZ;
+  const int z0 = (int)blockIdx.y * per;
+  const int nz = p.nz - z0 < per ? (int)(p.nz - z0) : per;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < nz) {
     // which redshifts of the block take the factor, and their powers of 1 + z
@@ -285,13 +287,30 @@ __global__ void __launch_bounds__(kBuildThreads, build_blocks(NB, INOUE, DZ)) bu
   }
 }
 
+// Redshifts per block: build_z where the grid then still holds two waves of
+// blocks; fewer on shorter redshift grids with Inoue14, which would leave SMs
+// idle behind the serial chain of a block.  QSO with Inoue14 (us, 16 to a block
+// / this rule / one thread per (z, pixel)): 8 redshifts 73 / 46 / 62, 16 97 / 50
+// / 60, 32 99 / 58 / 64, 64 103 / 77 / 83, 100 105 / 91 / 105, 300 163 / 161 /
+// 216.  Without it 4 to a block are within 8 us of the best at any length.
+static int build_per_block(const BuildParams& p, int nb, bool inoue, int nsm) {
+  const int most = build_z(inoue);
+  if (!inoue) return most;
+  const int64_t two_waves = 2 * (int64_t)nsm * build_blocks(nb, true, p.dbasis != nullptr);
+  const int64_t kz = p.nz * p.first[p.ngrid] / two_waves;
+  return kz < 1 ? 1 : kz < most ? (int)kz : most;
+}
+
 template <int NB>
-static int launch_build(const BuildParams& p, cudaStream_t stream) {
+static int launch_build(BuildParams& p, cudaStream_t stream) {
   bool igm = false;
   for (int g = 0; g < p.ngrid; ++g) igm = igm || p.g[g].igm;
   const bool inoue = igm && p.igm_model == RR_IGM_INOUE14;
-  const int kz = build_z(inoue);
-  dim3 grid((unsigned)p.first[p.ngrid], (unsigned)((p.nz + kz - 1) / kz));
+  int dev = 0, nsm = 0;
+  RR_CUDA_TRY(cudaGetDevice(&dev));
+  RR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  p.kz = build_per_block(p, NB, inoue, nsm);
+  dim3 grid((unsigned)p.first[p.ngrid], (unsigned)((p.nz + p.kz - 1) / p.kz));
   if (p.dbasis && inoue)
     build_basis_kernel<NB, true, true><<<grid, kBuildThreads, 0, stream>>>(p);
   else if (p.dbasis)

@@ -7,7 +7,7 @@ namespace rr {
 
 constexpr int kBuildGrids = 16;  // grids per launch
 
-// redshifts per block of the builder
+// redshifts per block of the builder, at most
 __host__ __device__ constexpr int build_z(bool inoue) { return inoue ? 16 : 4; }
 
 struct BuildGrid {
