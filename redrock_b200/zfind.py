@@ -50,7 +50,7 @@ from . import fitz as _fitz
 from . import _lib
 from .templates import parse_fulltype, solve_code
 from .engine import GridLayout, RowPack
-from .zscan import calc_zchi2_targets
+from .zscan import calc_zchi2_targets, scan_share
 
 MAX_VELO_DIFF = 1000.0
 MAX_VELO_DIFF_STAR = 100.0
@@ -400,9 +400,12 @@ class DeviceFitzPlan:
 
     Lazy one-time set-up (kernel attributes, constant tables) happens in an
     eager warm-up on the first target block before the first capture on a
-    device; the tile autotuner's choice is cached per batch shape."""
+    device; the tile autotuner's choice is cached per batch shape.  whole,
+    tail: of a rank's share of a batch (zscan.scan_share), else the local
+    targets are the whole batch."""
 
-    def __init__(self, local, templates, layout, nminima=3, nfine=15, graph=True):
+    def __init__(self, local, templates, layout, nminima=3, nfine=15, graph=True, whole=None,
+                 tail=None):
         import torch
         from . import autotune
         from .device import StatusWord, to_device
@@ -425,7 +428,8 @@ class DeviceFitzPlan:
         # so they share a workspace, made outside the graphs' memory pools
         # (in them it would be kept once per template: 7 GB for the seven)
         self.pair_ws = pair_workspace(self.rowpack, self.srcs, len(local) * self.K * nfine)
-        tail = few_tail(len(local))
+        self.whole = len(local) if whole is None else whole
+        self.tail = tail = few_tail(len(local)) if tail is None else tail
         key = _PackShape(layout, self.dbatch.batch.nblock, len(local))
         best = autotune.choice(key, self.bases, tail)
         if best is None and tail < len(local):
@@ -469,7 +473,8 @@ class DeviceFitzPlan:
     def _scan(self, dbatch):
         from .engine import TargetPack, run_fused
         pack = TargetPack(dbatch, status=self.status)
-        res, _ = run_fused(pack, self.bases, status=self.status, tiles=self.tiles)
+        res, _ = run_fused(pack, self.bases, status=self.status, tiles=self.tiles, tail=self.tail,
+                           ntarget=self.whole)
         return res
 
     def _fine(self, k, r, rowpack):
@@ -603,7 +608,7 @@ def zfind(targets, templates, mp_procs=1, nminima=3, archetypes=None, priors=Non
         from .priors import Priors
         priors = Priors(priors)
     comm = targets.comm
-    local = list(targets.local())
+    local, whole, tail = scan_share(targets)
     # wavegrids() is collective when the targets have a communicator: every
     # rank calls it, with or without local targets
     dwave = targets.wavegrids()
@@ -618,12 +623,13 @@ def zfind(targets, templates, mp_procs=1, nminima=3, archetypes=None, priors=Non
         # same target and template objects, so that a repeated call replays
         # the graph; like the packed-target cache it is keyed by identity
         from .zscan import _plan_cache
-        key = ("plan", layout.signature, nminima, nfine)
+        key = ("plan", layout.signature, nminima, nfine, whole, tail)
         plan = _plan_cache.get(key, list(local) + list(templates),
                                lambda: DeviceFitzPlan(local, templates, layout, nminima=nminima,
-                                                      nfine=nfine))
+                                                      nfine=nfine, whole=whole, tail=tail))
         plan.launch()
-        results = plan.coarse()
+        coarse = plan.coarse()
+        results = {t.id: coarse[t.id] for t in targets.local()}
         pres = _LazyFine(plan)
     elif chi2_scan is None:
         results = calc_zchi2_targets(targets, templates, mp_procs=mp_procs)

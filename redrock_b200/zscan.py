@@ -297,12 +297,29 @@ class _NoGC:
         return False
 
 
-def scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None):
+def scan_share(targets):
+    """(local targets in scan order, targets of the whole batch, how many of
+    the last local ones are in the batch's tail) of a DistTargets: which
+    kernel scans a target, and with it the last bits of its results, follows
+    the whole batch, so that they do not depend on how many ranks share it.
+    The tail is the last targets of all_target_ids that fill no block of the
+    fused scan (few_tail); on a rank its members come last."""
+    data = list(targets.local())
+    if targets.comm is None:
+        return data, len(data), few_tail(len(data))
+    ids = list(targets.all_target_ids)
+    tail = set(ids[len(ids) - few_tail(len(ids)):])
+    last = [t for t in data if t.id in tail]
+    return [t for t in data if t.id not in tail] + last, len(ids), len(last)
+
+
+def scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None, whole=None,
+                tail=None):
     """Fused scan of every target against every template (see
     _scan_device), with the cyclic garbage collector paused."""
     with _NoGC():
         out = _scan_device(targets, dtemplates, chunk=chunk, host=host,
-                           on_host_ready=on_host_ready)
+                           on_host_ready=on_host_ready, whole=whole, tail=tail)
     # bases built asynchronously (DistTemplate) report device errors here
     for dt in dtemplates:
         chk = getattr(dt, "check", None)
@@ -311,7 +328,8 @@ def scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None)
     return out
 
 
-def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None):
+def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None, whole=None,
+                 tail=None):
     """Fused scan of every target against every template.
 
     Returns a list (one entry per template) of results with zchi2 (T, nz),
@@ -323,7 +341,10 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     side stream while chunk k + 1 runs.  on_host_ready(hout) (host=True) is
     called once the GPU has the first two chunks queued, with the host
     result arrays (filled as the copies land, complete when this returns),
-    so that the caller can build its views of them meanwhile.
+    so that the caller can build its views of them meanwhile.  whole, tail:
+    the size of the batch that the targets are a rank's share of, and how
+    many of the last of them the few-target scan takes (scan_share); the
+    targets are the whole batch when not given.
     """
     layout = _layout_for(dtemplates[0], targets)
     all_bases = _bases_for(dtemplates, layout)
@@ -332,7 +353,8 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
         fused_ix = [i for i in range(len(all_bases)) if i not in plain_ix]
         out = [None] * len(all_bases)
         if fused_ix:
-            part = scan_device(targets, [dtemplates[i] for i in fused_ix], chunk=chunk, host=host)
+            part = scan_device(targets, [dtemplates[i] for i in fused_ix], chunk=chunk, host=host,
+                               whole=whole, tail=tail)
             for i, r in zip(fused_ix, part):
                 out[i] = r
         for i, r in zip(plain_ix, _bounded_scan(targets, [all_bases[i] for i in plain_ix],
@@ -350,9 +372,10 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
     st = StatusWord()
     bounds = _chunk_bounds(len(targets), chunk)
     # the last targets that fill no block, whatever chunk they fall into
+    whole = len(targets) if whole is None else whole
     few0 = len(targets)
     if all(b.stride == b.nbasis + b.nbasis % 2 for b in bases):
-        few0 -= few_tail(len(targets))
+        few0 -= few_tail(len(targets)) if tail is None else tail
     main = torch.cuda.current_stream()
     # consecutive chunks alternate between two compute streams, so that a
     # chunk's packing, y GEMMs and first scan launch need not wait for the
@@ -369,7 +392,7 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
         if few0 > 0 and yv in _lib.I8_VARIANTS:
             kpad = int(_lib.lib().rr_ygemm_kpad(layout.pix_stride))
             for b in bases:
-                if not y_in_scan(b, len(targets)):
+                if not y_in_scan(b, whole):
                     b.i8_digits(kpad, variant=yv)
         ev0 = torch.cuda.Event()
         ev0.record(main)
@@ -388,13 +411,12 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
                 pack = _pack_cache.get(("chunk", layout.signature, i0, len(sub)), sub,
                                        lambda: _pack_overlapped(sub, layout, st, cs))
             tiles = None
-            tail = max(0, i1 - max(i0, few0))
-            if AUTOTUNE and tail < len(sub):
+            few = max(0, i1 - max(i0, few0))
+            if AUTOTUNE and few < len(sub):
                 from . import autotune
-                tiles = autotune.tiles_of(autotune.choice(pack, bases, tail)
-                                          or autotune.tune(pack, bases, tail=tail))
-            res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=tail,
-                               ntarget=len(targets))
+                tiles = autotune.tiles_of(autotune.choice(pack, bases, few)
+                                          or autotune.tune(pack, bases, tail=few))
+            res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=few, ntarget=whole)
         keep.append((pack, res))
         if host:
             ev = torch.cuda.Event()
@@ -462,7 +484,7 @@ def calc_zchi2_targets(targets, templates, mp_procs=1, use_gpu=True):
     consistent.)
     """
     am_root = targets.comm is None or targets.comm.rank == 0
-    data = list(targets.local())
+    data, whole, tail = scan_share(targets)
     tids = [t.id for t in data]
     results = {tid: {} for tid in targets.local_target_ids()}
     if am_root:
@@ -482,7 +504,8 @@ def calc_zchi2_targets(targets, templates, mp_procs=1, use_gpu=True):
                                                        zcoeff=co[i])
     done = []
     out = scan_device(data, list(templates), host=True,
-                      on_host_ready=lambda hout: (fill(hout), done.append(True)))
+                      on_host_ready=lambda hout: (fill(hout), done.append(True)),
+                      whole=whole, tail=tail)
     if not done:
         fill(out)
     return results
