@@ -16,8 +16,9 @@ tiles (packed rows reused while in L2).
 ``tune(pack, bases)`` times the fused launch (CUDA events around the kernel
 alone, after one untimed run) for each candidate of every small-basis
 template present, keeps the fastest, and caches it per workload signature
-(grids, each small template's nbasis and redshift count, number of target
-blocks rounded up to a power of two).  ``choice`` returns the cached choice
+(grids, each small template's nbasis, redshift count and whether its y is
+summed in the scan, number of target blocks rounded up to a power of two).
+``choice`` returns the cached choice
 (or None).  Tuning runs the scan of the small templates a few times, so it
 belongs outside timed regions; the scan's results do not depend on the
 choice beyond rounding order within a thread (the tests check bit equality).
@@ -40,28 +41,35 @@ def _blocks(pack, tail):
     return pack.nblock if not tail else -(-(pack.ntarget - tail) // 32)
 
 
-def _key(pack, bases, tail):
-    small = tuple(sorted((b.nbasis, b.nz) for b in bases if b.nbasis in CANDIDATES))
+def _key(pack, bases, tail, ntarget):
+    from .engine import y_in_scan
+    n = pack.ntarget if ntarget is None else ntarget
+    # y in the scan is another kernel, with fewer registers to spare
+    small = tuple(sorted((b.nbasis, b.nz, y_in_scan(b, n)) for b in bases
+                         if b.nbasis in CANDIDATES))
+    large = tuple(sorted({y_in_scan(b, n) for b in bases if b.nbasis not in CANDIDATES}))
     nb = 1
     while nb < _blocks(pack, tail):
         nb *= 2
-    return (pack.layout.signature, small, nb)
+    return (pack.layout.signature, small, large, nb)
 
 
-def choice(pack, bases, tail=0):
-    return _cache.get(_key(pack, bases, tail))
+def choice(pack, bases, tail=0, ntarget=None):
+    return _cache.get(_key(pack, bases, tail, ntarget))
 
 
-def tune(pack, bases, repeats=1, tail=0):
+def tune(pack, bases, repeats=1, tail=0, ntarget=None):
     """Time the candidates and cache the fastest ZT per small nbasis.  tail:
     the pack's last targets that the few-target kernel takes (not timed: with
     one fused block of a 48-target batch QSO is fastest at two redshifts per
-    thread, with two at one)."""
+    thread, with two at one).  ntarget: the size of the whole batch when the
+    pack is a chunk of it, as in run_fused, so that the kernels timed are
+    those that will run."""
     from .engine import run_fused as _run
 
     def run_fused(*a, **kw):
-        return _run(*a, tail=tail, scan_tail=False, **kw)
-    key = _key(pack, bases, tail)
+        return _run(*a, tail=tail, ntarget=ntarget, scan_tail=False, **kw)
+    key = _key(pack, bases, tail, ntarget)
     if key in _cache:
         return _cache[key]
     best = {}

@@ -431,10 +431,10 @@ class DeviceFitzPlan:
         self.whole = len(local) if whole is None else whole
         self.tail = tail = few_tail(len(local)) if tail is None else tail
         key = _PackShape(layout, self.dbatch.batch.nblock, len(local))
-        best = autotune.choice(key, self.bases, tail)
+        best = autotune.choice(key, self.bases, tail, self.whole)
         if best is None and tail < len(local):
             pack0 = TargetPack(self.dbatch, status=self.status)
-            best = autotune.tune(pack0, self.bases, tail=tail)
+            best = autotune.tune(pack0, self.bases, tail=tail, ntarget=self.whole)
             del pack0
         self.tiles = autotune.tiles_of(best)
         dev = torch.cuda.current_device()

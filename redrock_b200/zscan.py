@@ -414,8 +414,9 @@ def _scan_device(targets, dtemplates, chunk=None, host=False, on_host_ready=None
             few = max(0, i1 - max(i0, few0))
             if AUTOTUNE and few < len(sub):
                 from . import autotune
-                tiles = autotune.tiles_of(autotune.choice(pack, bases, few)
-                                          or autotune.tune(pack, bases, tail=few))
+                tiles = autotune.tiles_of(
+                    autotune.choice(pack, bases, few, whole)
+                    or autotune.tune(pack, bases, tail=few, ntarget=whole))
             res, _ = run_fused(pack, bases, status=st, tiles=tiles, tail=few, ntarget=whole)
         keep.append((pack, res))
         if host:

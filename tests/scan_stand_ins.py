@@ -91,8 +91,8 @@ def install(monkeypatch):
         rec.log.append(("scan", rec.current.name, [t.id for t in pack.targets], tail, ntarget))
         return [_Result(len(pack.targets), b) for b in bases], status
 
-    def pack(targets, *a):
-        return types.SimpleNamespace(targets=list(targets), ntarget=len(targets),
+    def pack(targets, layout, *a):
+        return types.SimpleNamespace(targets=list(targets), ntarget=len(targets), layout=layout,
                                      nblock=max(1, -(-len(targets) // 32)))
 
     def bases_for(dts, layout):
