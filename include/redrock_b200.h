@@ -338,7 +338,7 @@ int rr_zscan_pairs(const rr_pair_template* tmpl, const rr_pair_segment* segs /* 
  * templates of a round's pairs are rebinned into it by the basis builder
  * first, so the sums stream.  Same results bit for bit, several times
  * faster.  rr_zscan_pairs_ws_bytes is the space for npairs pairs in one round
- * (SIZE_MAX: bad arguments); with less -- the space of two pairs at least --
+ * (SIZE_MAX: bad arguments); with less -- the space of one pair at least --
  * the call takes as many rounds as it needs. */
 size_t rr_zscan_pairs_ws_bytes(const rr_pair_segment* segs, int nseg, int32_t nbasis,
                                int64_t npairs);

@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kPairThreads)
   }
 }
 
-// workspace of one round: basis rows, M and y, flags (each 256-byte aligned)
+// workspace of one round: basis rows, M and y, flags
 struct PairsWsLayout {
   int64_t pix_stride = 0, per_pair = 0;
   int64_t off[kPairMaxSeg];
@@ -550,8 +550,8 @@ static int launch_pairs_ws(PairsParams p, const PairsWsLayout& w, unsigned char*
   return RR_OK;
 }
 
-// the call's rounds: an even number of pairs each (which keeps the arrays
-// aligned), nearly equal, within the builder's grid
+// the call's rounds: nearly equal, within the builder's grid (the arrays of any
+// number of pairs are aligned: basis rows are an even number of doubles)
 template <bool GRAD>
 static int run_pairs_ws(const PairsParams& p, const rr_pair_segment* segs, void* workspace,
                         size_t workspace_bytes, cudaStream_t st) {
@@ -559,12 +559,11 @@ static int run_pairs_ws(const PairsParams& p, const rr_pair_segment* segs, void*
       ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(p.rows)) & 15))
     return RR_EINVAL;
   const PairsWsLayout w = pairs_ws_layout(segs, p.nseg, p.tm.nbasis, GRAD);
-  int64_t most = (int64_t)(workspace_bytes / (size_t)w.per_pair) & ~(int64_t)1;
+  int64_t most = (int64_t)(workspace_bytes / (size_t)w.per_pair);
   if (most < 1) return RR_EINVAL;
   if (most > 65534 * build_z(false)) most = 65534 * build_z(false);
   const int64_t rounds = (p.npairs + most - 1) / most;
-  int64_t per_round = ((p.npairs + rounds - 1) / rounds + 1) & ~(int64_t)1;
-  if (per_round > most) per_round = most;
+  const int64_t per_round = (p.npairs + rounds - 1) / rounds;
   int rc = basis_tables(st);
   if (rc) return rc;
   unsigned char* ws = static_cast<unsigned char*>(workspace);

@@ -751,18 +751,18 @@ PAIR_WS_BYTES = 1 << 30
 
 
 def _pair_ws(nbytes, segs, nbasis, n, dev):
-    """Workspace of n pairs, at most PAIR_WS_BYTES (but two pairs); less, and
+    """Workspace of n pairs, at most PAIR_WS_BYTES (but one pair); less, and
     so more rounds, when the device has not that much left."""
-    need = int(nbytes(segs, len(segs), nbasis, n + n % 2))
-    two = int(nbytes(segs, len(segs), nbasis, 2))
-    size = min(need, max(two, PAIR_WS_BYTES))
+    need = int(nbytes(segs, len(segs), nbasis, n))
+    one = int(nbytes(segs, len(segs), nbasis, 1))
+    size = min(need, max(one, PAIR_WS_BYTES))
     while True:
         try:
             return torch.empty(size, dtype=torch.uint8, device=dev)
         except torch.cuda.OutOfMemoryError:
-            if size <= two:
+            if size <= one:
                 raise
-            size = max(two, size // 4)
+            size = max(one, size // 4)
 
 
 def pair_workspace(rowpack, sources, n):
