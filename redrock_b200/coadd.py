@@ -52,11 +52,15 @@ def coadd_targets(targets, cache_Rcsr=False, cosmics_nsig=0.):
             s0 = specs[0]
             npix = len(s0.wave)
             data0 = np.asarray(s0.R.data)
+            if data0.ndim != 2 or data0.shape[1] != npix:
+                raise ValueError("coadds need a resolution matrix of diagonals (scipy's DIA "
+                                 "format) as long as the wavelength grid")
             ndiag = data0.shape[0]
             first = len(exp_data)
             for s in specs:
                 d = np.asarray(s.R.data, dtype=np.float64)
-                if len(s.wave) != npix or d.shape != data0.shape:
+                if len(s.wave) != npix or d.shape != data0.shape or np.size(s.ivar) != npix \
+                        or np.size(s.flux) != npix:
                     raise ValueError("exposures on one wavelength grid must have the same "
                                      "length and resolution shape")
                 rdata.append(d.ravel())

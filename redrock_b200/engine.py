@@ -238,18 +238,26 @@ class DeviceBasis:
 # targets on the device
 # ---------------------------------------------------------------------------
 def spectrum_dia(s):
-    """(data[ndiag, npix], offsets[ndiag]) of a redrock Spectrum's R."""
+    """(data[ndiag, npix], offsets[ndiag]) of a redrock Spectrum's R.  Columns
+    that the matrix leaves out at its end (scipy's todia() stops at the last
+    stored one) are zero, as scipy reads them."""
     npix = len(s.wave)
+
+    def whole(data, offsets):
+        d = np.asarray(data)[:, :npix]
+        if d.shape[1] < npix:
+            d = np.pad(d, ((0, 0), (0, npix - d.shape[1])))
+        return d, np.asarray(offsets)
     R = getattr(s, "R", None)
     if R is None and getattr(s, "_mpshared", False):
-        return np.asarray(s.R_data)[:, :npix], np.asarray(s.R_offsets)
+        return whole(s.R_data, s.R_offsets)
     if R is None:
         R = getattr(s, "_Rcsr", None)
     if R is None:
         raise ValueError("spectrum has no resolution matrix")
     if not hasattr(R, "offsets"):
         R = R.todia()
-    return np.asarray(R.data)[:, :npix], np.asarray(R.offsets)
+    return whole(R.data, R.offsets)
 
 
 class TargetBatch:
@@ -293,7 +301,7 @@ class TargetBatch:
             for s, (g, sl) in zip(t.spectra, assign):
                 d, o = spectrum_dia(s)
                 npix = len(s.wave)
-                if npix != layout.npix[g]:
+                if npix != layout.npix[g] or np.size(s.ivar) != npix or np.size(s.flux) != npix:
                     raise ValueError("spectrum length does not match its wavelength grid")
                 wide = np.abs(o) > _lib.HALF_BAND
                 if np.any(wide) and np.any(d[wide] != 0):
@@ -941,6 +949,8 @@ class PlainTarget:
             weights = np.concatenate([s.ivar for s in spectra])
             flux = np.concatenate([s.flux for s in spectra])
             wflux = weights * flux
+        if not len(weights) == len(flux) == len(wflux) == self.npix:
+            raise ValueError("weights and flux must have the spectra's number of pixels")
         self.w = to_device(weights)
         self.flux = to_device(flux)
         self.wflux = to_device(wflux)
