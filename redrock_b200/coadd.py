@@ -31,7 +31,7 @@ import torch
 
 from . import _lib
 from .device import StatusWord, device, ptr, stream_handle, struct_bytes, to_device
-from .engine import _concat
+from .engine import GATHER_BYTES, _concat
 
 
 def _groups(target):
@@ -85,8 +85,10 @@ def coadd_targets(targets, cache_Rcsr=False, cosmics_nsig=0.):
     # gathered straight into pinned memory for the upload
     pinned = {}
 
+    threads = d_off * 8 >= GATHER_BYTES
+
     def up(name, parts):
-        a = _concat(parts, np.float64, pinned, name)
+        a = _concat(parts, np.float64, pinned, name, threads)
         t = pinned.get(name)
         return to_device(a) if t is None else t.to(dev, non_blocking=True)
     drd, div, dfl = up("rdata", rdata), up("ivar", ivar), up("flux", flux)

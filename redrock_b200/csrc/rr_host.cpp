@@ -1,10 +1,11 @@
 // Host side of the target uploads: the arrays of a batch (hundreds of
 // resolution matrices, 0.2 MB each) gathered into one pinned buffer.
 //
-// One core copies at about 6 GB/s into pinned memory -- 14 ms for 100 DESI
-// targets, half of fitz's time for them -- while the memory of the machine
-// takes several times that, so batches of 4 MB and more are split into equal
-// byte ranges over up to kMaxThreads threads that live for the call.
+// One core copies at about 6 GB/s into pinned memory -- 11 to 14 ms for 100
+// DESI targets, half of fitz's time for them -- while the memory of the machine
+// takes several times that, so arrays of 4 MB and more are split into equal
+// byte ranges over up to kMaxThreads threads that live for the call (the
+// callers come here for batches of 16 MB and more).
 #include <algorithm>
 #include <cstdint>
 #include <cstring>

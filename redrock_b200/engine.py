@@ -325,13 +325,14 @@ class TargetBatch:
         # the large arrays are gathered straight into pinned host memory (when
         # a GPU is present), so their upload needs no second staging copy
         self._pinned = {}
+        threads = data_off * 8 >= GATHER_BYTES
         self.rdata = _concat([np.asarray(d, dtype=np.float64).ravel() for d in rdata], np.float64,
-                             self._pinned, "rdata")
+                             self._pinned, "rdata", threads)
         self.roffs = _concat([np.asarray(o, dtype=np.int32) for o in roffs], np.int32)
         self.ivar = _concat([np.asarray(v, dtype=np.float64) for v in ivar], np.float64,
-                            self._pinned, "ivar")
+                            self._pinned, "ivar", threads)
         self.flux = _concat([np.asarray(v, dtype=np.float64) for v in flux], np.float64,
-                            self._pinned, "flux")
+                            self._pinned, "flux", threads)
 
     def host_arrays(self):
         return (self.descs, self.segs_bytes, self.first, self.rows, self.rdata, self.roffs,
@@ -345,10 +346,19 @@ class TargetBatch:
         return DeviceTargetBatch(self)
 
 
-def _concat(parts, dtype, pinned=None, name=None):
+# bytes of resolution data from which a batch's arrays are gathered by threads
+# (rr_host_gather).  For fewer, collecting the addresses, starting the threads
+# and uploading from several caches cost what the copies save; fitz of STAR
+# minima, ms copied here / gathered (median): 4 targets (2.8 MB) 2.17 / 2.22, 8
+# 2.83 / 2.93, 12 3.34 / 4.53, 16 (11 MB) 4.08 / 5.04, 24 (17 MB) 5.12 / 4.96, 32
+# 6.65 / 5.70, 64 13.2 / 10.1, 100 20.3 / 14.1
+GATHER_BYTES = 16 << 20
+
+
+def _concat(parts, dtype, pinned=None, name=None, threads=False):
     """Concatenate 1-D arrays; into a pinned host tensor (kept in
     pinned[name]) when pinned is given, the result is >= 1 MB and a GPU is
-    present."""
+    present, and then by several threads if asked for."""
     dt = np.dtype(dtype)
     n = sum(p.size for p in parts)
     if pinned is not None and n * dt.itemsize >= (1 << 20) and torch.cuda.is_available():
@@ -356,7 +366,7 @@ def _concat(parts, dtype, pinned=None, name=None):
                         pin_memory=True)
         pinned[name] = t
         out = t.numpy()
-        if all(p.dtype == dt and p.flags.c_contiguous for p in parts):
+        if threads and all(p.dtype == dt and p.flags.c_contiguous for p in parts):
             src = np.array([p.ctypes.data for p in parts], dtype=np.uintp)
             size = np.array([p.nbytes for p in parts], dtype=np.int64)
             rc = _lib.lib().rr_host_gather(src.ctypes.data, size.ctypes.data, len(parts),
