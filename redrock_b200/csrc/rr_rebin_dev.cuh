@@ -471,7 +471,7 @@ __device__ __forceinline__ bool div_range_b(double b) {
 // order, each sample read once.  j is first_above(e_lo).  Returns false
 // when the bin falls outside the input range; exact is false when a division
 // was out of div_near's range and res is not to be used.  With DZ, dres gets
-// dT/dz from the edge values, as in rebin_bin_strided (to a rounding or two).
+// dT/dz from the edge values, as in rebin_bin_strided.
 template <int NB, bool DZ = false>
 __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int64_t nx,
                                               const double* __restrict__ y, int64_t ystride,
@@ -550,7 +550,10 @@ __device__ __forceinline__ bool rebin_bin_reg(const double* __restrict__ x, int6
   for (int b = 0; b < NB; ++b) {
     ok = ok & div_range(res[b]);
     res[b] = div_near(res[b], width, r);
-    if (DZ) dres[b] = (res[b] - dres[b] * r) / zp1;
+    if (DZ) {
+      ok = ok & div_range(dres[b]);
+      dres[b] = (res[b] - div_near(dres[b], width, r)) / zp1;
+    }
   }
   exact = ok;
   return true;
