@@ -30,11 +30,15 @@ constexpr int pair_stride() { return (NB & 1) ? NB : NB + 1; }
 
 template <int NB>
 struct PairSmem {
+  // sums at a time: M and y, or the gradient pass's 3 + 2 NB, which are more
+  // for one and two bases
+  static constexpr int kGram = NB * (NB + 1) / 2 + NB;
+  static constexpr int kSum = kGram > 3 + 2 * NB ? kGram : 3 + 2 * NB;
   double t[kPairThreads * pair_stride<NB>()];  // basis rows of the chunk + halo
   double dt[kPairThreads * pair_stride<NB>()]; // their z derivatives (gradient mode)
   double xs[kPairWin];                          // staged template wavelengths
   double ys[NB * kPairWin];                     // staged template fluxes
-  double red[kPairThreads / 32][NB * (NB + 1) / 2 + NB];
+  double red[kPairThreads / 32][kSum];
   double c[NB];
   int64_t jlo, jhi, win;
   int fix;

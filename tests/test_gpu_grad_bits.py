@@ -14,7 +14,9 @@ pytestmark = [pytest.mark.gpu,
 
 @pytest.mark.parametrize("nb,igm,extreme", [(10, "None", False), (4, "Inoue14", False),
                                             (5, "None", True), (3, "Inoue14", True),
-                                            (7, "Calura12", True)])
+                                            (7, "Calura12", True),
+                                            # more gradient sums than M and y
+                                            (1, "Inoue14", True), (2, "None", False)])
 def test_gradients_are_the_same_bits(nb, igm, extreme):
     import torch
     from redrock_b200 import _lib, synth, targets as T
