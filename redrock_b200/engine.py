@@ -702,7 +702,8 @@ def run_fused(pack, bases, stream=None, status=None, ygemm=None, kernel_events=N
             _record(e1, stream)
             kernel_events.append((e0, e1))
     for r in results[:1]:
-        r.few = (few, rows)   # outlive the launches
+        # outlive the launches; not the FewRows itself, which holds the pack
+        r.few = (None if few is None else few.lrows, rows)
     run_fused.last_counter = counter
     return results, st
 

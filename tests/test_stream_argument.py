@@ -1,13 +1,19 @@
 """Calls given a stream of their own (CPU, with stand-ins for the library and
 the streams): the buffers they make are ready before the launches on that
 stream read or write them, and are kept from reuse until it is done."""
+import gc
 import types
+import weakref
 
 import numpy as np
 import pytest
 import torch
 
 from redrock_b200 import _lib, engine
+
+
+class _Pack(types.SimpleNamespace):
+    pass
 
 
 class _Stream:
@@ -97,7 +103,7 @@ def test_scan_tail(calls, n, tail):
     log, main, side = calls
     layout = types.SimpleNamespace(signature=(), pix_stride=64)
     nblock = -(-n // 32)
-    pack = types.SimpleNamespace(
+    pack = _Pack(
         ntarget=n, nblock=nblock, layout=layout, rw=torch.zeros(1),
         rows=torch.arange(32 * nblock, dtype=torch.int32),
         scan_targets_struct=lambda nb=None, rows=None: _lib.ScanTargets(
@@ -105,10 +111,15 @@ def test_scan_tail(calls, n, tail):
     basis = types.SimpleNamespace(layout=layout, method=_lib.RR_SOLVE_PCA, stride=2, nbasis=1,
                                   nz=3, basis=torch.zeros(2), prior=None, oii=None)
     res, _ = engine.run_fused(pack, [basis], stream=side, status=_st(), ygemm="fp64", tail=tail)
-    few, rows = res[0].few
+    lrows, rows = res[0].few
     held, args = _check(log, "rr_pack_few")
-    assert few.lrows.data_ptr() in held & args
+    assert lrows.data_ptr() in held & args
     if n > tail:
         held, _ = _check(log, "rr_zscan_fused")
         assert rows.data_ptr() in held
         assert rows[n - tail:].eq(-1).all() and rows[:n - tail].ge(0).all()
+    # results a caller keeps do not keep the packed targets (0.8 MB each)
+    ref = weakref.ref(pack)
+    del pack
+    gc.collect()
+    assert ref() is None and res
