@@ -9,7 +9,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 #include "../../include/redrock_b200.h"
@@ -48,13 +48,14 @@ extern "C" int rr_host_gather(const void* const* src, const int64_t* bytes, int6
   std::thread th[kMaxThreads];
   const int64_t per = (total / k + 63) & ~(int64_t)63;
   int started = 0;
-  // the last range, and those whose thread the system refuses, are this
-  // thread's own
+  // the last range, and those whose thread the system refuses or has no memory
+  // for, are this thread's own: nothing may leave a C entry, least of all past
+  // threads that still run
   int64_t rest = 0;
   try {
     for (; started + 1 < k && rest + per < total; ++started, rest += per)
       th[started] = std::thread(copy_range, src, bytes, n, out, rest, rest + per);
-  } catch (const std::system_error&) {
+  } catch (const std::exception&) {
   }
   copy_range(src, bytes, n, out, rest, total);
   for (int i = 0; i < started; ++i) th[i].join();
