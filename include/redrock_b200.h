@@ -334,7 +334,9 @@ int rr_zscan_pairs(const rr_pair_template* tmpl, const rr_pair_segment* segs /* 
                    int64_t npairs, double* chi2, double* coeff /* [npairs][nbasis] */,
                    double* penalty /* [npairs] or NULL */, int* status, rr_stream_t stream);
 
-/* The same pair scan in rounds through a workspace (16-byte aligned): the
+/* The same pair scan in rounds through a workspace (16-byte aligned), which is
+ * the one the Python package calls (rr_zscan_pairs and rr_zscan_pairs_grad are
+ * for callers that have no workspace to give): the
  * templates of a round's pairs are rebinned into it by the basis builder
  * first, so the sums stream.  Same results bit for bit, several times
  * faster.  rr_zscan_pairs_ws_bytes is the space for npairs pairs in one round

@@ -159,7 +159,7 @@ static __device__ __noinline__ double transmission_slope(double t, double z, dou
 // memory as whole 16-byte columns of a warp's 32 consecutive rows.
 // Per (z, pixel, basis) about 35 FP64 operations at two samples to a bin (135
 // with three full divisions).  Bound by its sample loads: L1 77 % busy, the
-// FP64 pipe 46 %.  GALAXY, 3311 x 7958 x 10: 3.60 -> 1.86 ms; QSO with
+// FP64 pipe 46 % (QSO with Inoue14 45 and 47 %: latency).  GALAXY, 3311 x 7958 x 10: 3.60 -> 1.86 ms; QSO with
 // Inoue14, 3794 x 7958 x 4: 2.14 -> 1.24 ms (build_basis_any_kernel, one
 // thread per (z, pixel), before).
 constexpr int kBuildThreads = 128;

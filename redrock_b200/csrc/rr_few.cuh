@@ -32,10 +32,12 @@
 // Measured (DESI grids): 1 target x GALAXY, QSO and 5 STAR templates, from host
 // arrays, 20.4 -> 2.0 ms (kernels 19.5 -> 1.1 ms); per target of a pair GALAXY
 // 0.53, QSO 0.23, STAR 0.04 ms (0.92, 0.40, 0.34 with a whole warp per (target,
-// z) and no sharing); 37 targets, 32 of them fused, 41.8 -> 29.2 ms; 7 targets x
-// a 5-vector NMF template of 3311 redshifts 15.4 -> 5.3 ms against the plain
-// chain.  The FP64 pipe is 47 % busy on GALAXY: the warps wait for
-// shared-memory reads that 255 registers leave no room to start earlier.
+// z) and no sharing); 37 targets, 32 of them fused, 41.8 -> 26.0 ms.  A 5-vector
+// NMF template of 3311 redshifts, against the plain chain: 1 target 2.3 -> 1.5
+// ms, 7 targets 15.4 -> 5.2, 32 69 -> 21, 100 218 -> 64, 256 559 -> 159.  The FP64
+// pipe is 42 % busy on GALAXY with one target and 49 % with two: the warps wait
+// for shared-memory reads that 255 registers leave no room to start earlier
+// (NMF: L1 73 %, FP64 36 %).
 #pragma once
 #include <cmath>
 #include <cstring>

@@ -18,7 +18,9 @@
 // from shared rows i..i+10.  Template samples covering the chunk are staged
 // in shared memory first, so the per-pixel search for the first sample
 // beyond a bin edge runs on shared memory.  rr_zscan_pairs_ws
-// (rr_pairs_ws.cu) does the same in rounds through a workspace.
+// (rr_pairs_ws.cu) does the same in rounds through a workspace, several times
+// faster; the Python package calls that one, and this is for C callers that
+// have no workspace to give.
 #include "rr_pairs.cuh"
 
 namespace rr {

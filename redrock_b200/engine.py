@@ -543,7 +543,9 @@ def y_in_scan(basis, ntarget):
     1000 targets.  The scan sums y at 13 TFMA/s; ten bases leave it no
     registers for y and pay about twice that.  With the GEMM and without, ms:
     32 targets GALAXY 10.96 / 11.97, QSO 5.43 / 5.35, STAR 2.81 / 1.90; 64
-    targets QSO 9.89 / 10.04; 128 targets STAR 4.32 / 3.46."""
+    targets QSO 9.89 / 10.04; 128 targets STAR 4.32 / 3.46.  ntarget is the
+    whole batch with its tail, so 33 to 52 targets count as two blocks though
+    the fused scan has one (there QSO takes the GEMM, 1.5 % slower)."""
     L = _lib.lib()
     kpad = int(L.rr_ygemm_kpad(basis.layout.pix_stride))
     tiles = -(-basis.nz // (80 // basis.nbasis)) * -(-ntarget // 128)
@@ -578,7 +580,10 @@ def _record(ev, stream):
 # fused scan go through the few-target kernel when there are at most this
 # many of them: with all seven templates a target costs it 0.80 ms (GALAXY
 # 0.53, QSO 0.23, STAR 0.04), a block of the fused scan 16 to 18 ms however
-# many of its lanes are used (GALAXY 10.5, QSO 4.2 to 7.9, STAR 2.6)
+# many of its lanes are used (GALAXY 10.5, QSO 4.2 to 7.9, STAR 2.6).  One
+# number for every set of templates, so that a target's sums do not depend on
+# the set: GALAXY or QSO alone cross at about the same number, STAR alone would
+# at more than 31 (calls of 20 and 21 STAR targets 3.2 and 5.0 ms)
 FEW_MAX = 20
 
 
