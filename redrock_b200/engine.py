@@ -355,10 +355,11 @@ class TargetBatch:
 GATHER_BYTES = 16 << 20
 
 
-def _concat(parts, dtype, pinned=None, name=None, threads=False):
+def _concat(parts, dtype, pinned=None, name=None, threads=None):
     """Concatenate 1-D arrays; into a pinned host tensor (kept in
     pinned[name]) when pinned is given, the result is >= 1 MB and a GPU is
-    present, and then by several threads if asked for."""
+    present, and then by several threads if threads (None: if the result has
+    GATHER_BYTES; a batch's smaller arrays follow its resolution data)."""
     dt = np.dtype(dtype)
     n = sum(p.size for p in parts)
     if pinned is not None and n * dt.itemsize >= (1 << 20) and torch.cuda.is_available():
@@ -366,6 +367,8 @@ def _concat(parts, dtype, pinned=None, name=None, threads=False):
                         pin_memory=True)
         pinned[name] = t
         out = t.numpy()
+        if threads is None:
+            threads = out.nbytes >= GATHER_BYTES
         if threads and all(p.dtype == dt and p.flags.c_contiguous for p in parts):
             src = np.array([p.ctypes.data for p in parts], dtype=np.uintp)
             size = np.array([p.nbytes for p in parts], dtype=np.int64)
