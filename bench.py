@@ -592,7 +592,7 @@ def adjoint_study(rtg, tms, torch):
         npairs += len(pz)
     return {"pairs": npairs, "ms": ms, "value": npairs / (ms / 1e3),
             "unit": "gradient evals/s (chi2, dchi2/dz, d2chi2/dz2, dchi2/dflux per (target, z))",
-            "kernel": "zscan_pairs_kernel<NB, grad> (template rebinned + IGM per pair)"}
+            "kernel": "build_basis_kernel with dT/dz, then pairs_sums_kernel<NB, grad>"}
 
 
 def archetype_study(tg, rtg, torch, narch=24):
